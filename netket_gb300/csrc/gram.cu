@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "chol_tc.cuh"
 #include "gram_tc.cuh"
+#include "signsum.cuh"
 
 namespace vmck {
 
@@ -34,57 +35,10 @@ __global__ void sign_bits_kernel(const int8_t *__restrict__ x, int64_t n, int N,
   bits[e] = v;
 }
 
-// g_s = t_s . (tbar + x_s^T Kbar) + x_s . xbar  (FP64); 16 samples per CTA,
-// their configurations staged once in shared memory (N <= 288).
+// g_s = O(s) . obar = t_s . (tbar + x_s^T Kbar) + x_s . xbar: FP64 t through
+// o_v_f64, FP32 t below; 16 samples per CTA, their configurations staged once in
+// shared memory (N <= 288).
 constexpr int G_SPB = 16, G_NMAX = 288;
-
-template <typename T>
-__global__ void __launch_bounds__(256) g_vector_kernel(const T *__restrict__ t,
-                                                       const int8_t *__restrict__ x, int N, int M,
-                                                       int64_t n, const double *__restrict__ obar,
-                                                       double *__restrict__ g) {
-  __shared__ int8_t xs[G_SPB][G_NMAX];
-  __shared__ double part[G_SPB][8];
-  const int64_t s0 = (int64_t)blockIdx.x * G_SPB;
-  const double *tbar = obar, *Kbar = obar + M, *xbar = obar + M + (int64_t)N * M;
-  const int ns = (int)std::min<int64_t>(G_SPB, n - s0);
-  for (int e = threadIdx.x; e < G_SPB * N; e += blockDim.x) {
-    int q = e / N, i = e % N;
-    xs[q][i] = (q < ns) ? x[(s0 + q) * N + i] : int8_t(0);
-  }
-  __syncthreads();
-  double gp[G_SPB];
-#pragma unroll
-  for (int q = 0; q < G_SPB; ++q) gp[q] = 0;
-  for (int j = threadIdx.x; j < M; j += blockDim.x) {
-    double y[G_SPB];
-    const double tb = tbar[j];
-#pragma unroll
-    for (int q = 0; q < G_SPB; ++q) y[q] = tb;
-    for (int i = 0; i < N; ++i) {
-      const double kb = Kbar[(int64_t)i * M + j];
-#pragma unroll
-      for (int q = 0; q < G_SPB; ++q) y[q] += xs[q][i] > 0 ? kb : -kb;
-    }
-#pragma unroll
-    for (int q = 0; q < G_SPB; ++q)
-      if (q < ns) gp[q] += (double)t[(s0 + q) * M + j] * y[q];
-  }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < G_SPB; ++q) {
-    double v = warp_sum(gp[q]);
-    if (lane == 0) part[q][wid] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < ns) {
-    const int q = threadIdx.x;
-    double v = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += part[q][w];
-    for (int i = 0; i < N; ++i) v += xs[q][i] > 0 ? xbar[i] : -xbar[i];
-    g[s0 + q] = v;
-  }
-}
 
 // Double-float form for FP32 tanh(theta): the ~6.5e8 accumulations per call
 // would otherwise run on the FP64 pipe.  t enters as c + s0 (the shifted,
@@ -458,8 +412,8 @@ extern "C" int vmck_rbm_gram(vmck_ctx *ctx, vmck_stream s, int32_t mode, int32_t
   if (rc) return rc;
   const unsigned gblocks = (unsigned)((n + G_SPB - 1) / G_SPB);
   if (dtype == VMCK_F64) {
-    g_vector_kernel<double><<<gblocks, 256, 0, st>>>(static_cast<const double *>(tanh_theta), x,
-                                                     N, M, n, obar, w.g);
+    if ((rc = o_v_f64(st, static_cast<const double *>(tanh_theta), x, N, M, n, obar, w.g)))
+      return rc;
   } else {
     const int terms = mode == 2 ? 2 : (mode == 3 ? 1 : (mode == 4 ? 3 : 0));
     gram_shift_kernel<<<ceil_div(n * (int64_t)M, 256), 256, 0, st>>>(

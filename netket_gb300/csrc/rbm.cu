@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "localop.cuh"
 #include "pauli.cuh"
+#include "signsum.cuh"
 
 namespace vmck {
 
@@ -642,6 +643,8 @@ extern "C" int vmck_rbm_o_v(vmck_stream s, int32_t dtype, const void *tanh_theta
   VMCK_REQUIRE(tanh_theta && x && v && out && N > 0 && M > 0 && n >= 0, "rbm_o_v arguments");
   if (n == 0) return VMCK_OK;
   const unsigned grid = (unsigned)((n + 7) / 8);
+  if (dtype == VMCK_F64 && signed_rows_fit(N))
+    return o_v_f64(as_stream(s), static_cast<const double *>(tanh_theta), x, N, M, n, v, out);
   if (dtype == VMCK_F64)
     o_v_kernel<double><<<grid, 256, 0, as_stream(s)>>>(static_cast<const double *>(tanh_theta), x,
                                                         N, M, n, v, out);
@@ -660,6 +663,10 @@ extern "C" int vmck_rbm_logpsi(vmck_stream s, int32_t dtype, const void *params,
                                void *theta_out, void *tanh_out) {
   VMCK_REQUIRE(params && x && logpsi && N > 0 && M > 0 && n >= 0, "rbm_logpsi arguments");
   if (n == 0) return VMCK_OK;
+  if (dtype == VMCK_F64 && signed_rows_fit(N))
+    return logpsi_f64(as_stream(s), static_cast<const double *>(params), N, M, x, n,
+                      static_cast<double *>(logpsi), static_cast<double *>(theta_out),
+                      static_cast<double *>(tanh_out));
   if (dtype == VMCK_F64)
     return launch_logpsi<double>(as_stream(s), params, N, M, x, n, logpsi, theta_out, tanh_out);
   if (dtype == VMCK_F32)
@@ -724,8 +731,9 @@ static int64_t ot_chunk(int64_t n) { return 1024; }
 
 extern "C" int64_t vmck_ot_v_workspace_size(int32_t N, int32_t M, int64_t n) {
   int64_t P = (int64_t)M + (int64_t)N * M + N;
-  int64_t nchunk = (n + ot_chunk(n) - 1) / ot_chunk(n);
-  if (nchunk < 1) nchunk = 1;
+  if (N <= 0 || M <= 0 || n <= 0) return P;
+  const int64_t nchunk = std::max<int64_t>((n + ot_chunk(n) - 1) / ot_chunk(n),
+                                           ot_v_f64_chunks(N, M, n));
   return nchunk * P;
 }
 
@@ -736,20 +744,21 @@ extern "C" int vmck_rbm_ot_v(vmck_stream s, int32_t dtype, const void *tanh_thet
                "rbm_ot_v arguments");
   VMCK_REQUIRE(workspace_len >= vmck_ot_v_workspace_size(N, M, n), "rbm_ot_v workspace too small");
   const int64_t chunk = ot_chunk(n);
-  const int nchunk = (int)((n + chunk - 1) / chunk);
+  int nchunk = (int)((n + chunk - 1) / chunk);
   dim3 grid((M + OT_TJ - 1) / OT_TJ, (N + OT_TI - 1) / OT_TI, nchunk);
   cudaStream_t st = as_stream(s);
-  if (dtype == VMCK_F64)
-    ot_v_partial_kernel<double><<<grid, 256, 0, st>>>(static_cast<const double *>(tanh_theta), x,
-                                                      N, M, n, chunk, v, workspace);
-  else if (dtype == VMCK_F32)
+  int rc;
+  if (dtype == VMCK_F64) {
+    nchunk = ot_v_f64_chunks(N, M, n);
+    rc = ot_v_f64(st, static_cast<const double *>(tanh_theta), x, N, M, n, v, workspace);
+  } else if (dtype == VMCK_F32) {
     ot_v_partial_kernel<float><<<grid, 256, 0, st>>>(static_cast<const float *>(tanh_theta), x, N,
                                                      M, n, chunk, v, workspace);
-  else {
+    rc = check_launch("rbm_ot_v partial");
+  } else {
     set_last_error("rbm_ot_v: dtype %d unsupported", dtype);
     return VMCK_ERR_UNSUPPORTED;
   }
-  int rc = check_launch("rbm_ot_v partial");
   if (rc) return rc;
   const int64_t P = (int64_t)M + (int64_t)N * M + N;
   reduce_chunks_kernel<<<ceil_div(P, 256), 256, 0, st>>>(workspace, P, nchunk, out);
