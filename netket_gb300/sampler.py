@@ -206,12 +206,19 @@ class MetropolisSampler:
             state = self.init_state(machine, params)
         N = self.hilbert.size
         M = machine.sizes_from_flat(params.numel(), N)
-        if self.reset_chains:
-            state.σ = self.hilbert.random_state(state.seed, self.n_chains,
-                                                stream_id=2 + state.counter)
+        state = self._restart(state)
         from .kernels import rbm_forward
         lp, _, _ = rbm_forward(params, state.σ, N, M)
         state.log_prob = 2.0 * lp.to(torch.float64)
+        return state
+
+    def _restart(self, state):
+        """``reset`` of an existing state without the log-probabilities, which a
+        sampling call that follows writes for its own final configurations."""
+        if self.reset_chains:
+            state.σ = self.hilbert.random_state(state.seed, self.n_chains,
+                                                stream_id=2 + state.counter)
+        state.log_prob = torch.empty_like(state.log_prob)
         state.n_accepted_proc = torch.zeros_like(state.n_accepted_proc)
         state.n_steps_proc = 0
         return state
