@@ -247,271 +247,6 @@ __global__ void batch_advance_counters_kernel(vmck_batch_chains *inst, int n_ins
   if (i < n_inst) inst[i].counter += (uint64_t)steps * (uint64_t)inst[i].sweep_size;
 }
 
-// ------------------------------------------------------------ Exchange, W in L2
-constexpr int XS_MAXDEG = 16;  // incident clusters kept per site; more: full recounts
-
-__device__ __forceinline__ int warp_sum_int(int v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Position of the n-th (0-based) set bit of v, which has more than n set bits:
-// a bisection on popcounts of the low half, quarter, ... of what is left.
-__device__ __forceinline__ int nth_set_bit(uint32_t v, int n) {
-  int pos = 0, c = __popc(v & 0xFFFFu);
-  if (n >= c) { n -= c; pos += 16; v >>= 16; }
-  c = __popc(v & 0xFFu);
-  if (n >= c) { n -= c; pos += 8; v >>= 8; }
-  c = __popc(v & 0xFu);
-  if (n >= c) { n -= c; pos += 4; v >>= 4; }
-  c = __popc(v & 0x3u);
-  if (n >= c) { n -= c; pos += 2; v >>= 2; }
-  if (n >= (int)(v & 1u)) pos += 1;
-  return pos;
-}
-
-// Exchange chains of an FP32 RBM whose weights do not fit in shared memory (those
-// that do: sampler_filter.cu): W, b, a are read through L2 (2 MB for N = 256, M = 2048) and theta
-// lives in the warp's shared memory (M floats); log_cosh(theta) is recomputed
-// where it is needed instead of stored (the same function of the same value,
-// so the same bits), and an accepted move recomputes theta'.  A chain then
-// holds ~8.3 KB of shared memory and few registers: 24 chains per SM at
-// M = 2048, where metropolis_kernel's four M-vectors leave 4 (a version with
-// theta in registers, 64 per lane, was register-bound at 16 and stalled on the
-// L2 loads of W: 25 % warps active).  Warps loop over chains (b += gridDim.x
-// wpb).  Random stream, proposal order and every floating-point expression
-// match metropolis_kernel<float, 1>, so the samples are identical.
-constexpr int XL_WARPS = 24;
-
-__global__ void __launch_bounds__(32 * XL_WARPS, 1) metropolis_exchange_l2_kernel(
-    const float *__restrict__ params, int N, int M, int8_t *sigma, double *log_prob,
-    int64_t *n_accepted, int B, int sweep, int n_discard, int L, int8_t *samples, uint32_t k0,
-    uint32_t k1, uint64_t counter, const int32_t *__restrict__ clusters, int C) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int nwords = (C + 31) >> 5;
-  const float *Wg = params + M, *bg = params, *ag = params + M + (int64_t)N * M;
-  float *logtab = reinterpret_cast<float *>(smem_raw);                // C + 1
-  int16_t *cl = reinterpret_cast<int16_t *>(logtab + C + 1);          // 2C
-  int16_t *inc = cl + 2 * C;                                          // N x XS_MAXDEG
-  int *deg = reinterpret_cast<int *>(                                 // N
-      (reinterpret_cast<uintptr_t>(inc + (size_t)N * XS_MAXDEG) + 3) & ~uintptr_t(3));
-  __shared__ int overflow;
-  unsigned char *per_warp_base = reinterpret_cast<unsigned char *>(
-      (reinterpret_cast<uintptr_t>(deg + N) + 15) & ~uintptr_t(15));
-  const size_t per_warp = 4 * (size_t)M + (((size_t)N + 15) & ~size_t(15)) + 4 * (size_t)nwords;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int wpb = (int)(blockDim.x >> 5);
-  {  // clusters and incidence lists
-    for (int i = tid; i < N; i += blockDim.x) deg[i] = 0;
-    for (int k = tid; k <= C; k += blockDim.x) logtab[k] = logf((float)k);
-    for (int q = tid; q < 2 * C; q += blockDim.x) cl[q] = (int16_t)clusters[q];
-    if (tid == 0) overflow = 0;
-    __syncthreads();
-    for (int q = tid; q < C; q += blockDim.x) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int site = cl[2 * q + e];
-        const int pos = atomicAdd(&deg[site], 1);
-        if (pos < XS_MAXDEG) inc[site * XS_MAXDEG + pos] = (int16_t)q;
-        else overflow = 1;
-      }
-    }
-    __syncthreads();
-  }
-  const bool full_recount = overflow != 0;
-  float *ths = reinterpret_cast<float *>(per_warp_base + warp * per_warp);  // theta, M
-  int8_t *xs = reinterpret_cast<int8_t *>(ths + M);
-  uint32_t *mask = reinterpret_cast<uint32_t *>(xs + ((N + 15) & ~15));
-  for (int b = blockIdx.x * wpb + warp; b < B; b += gridDim.x * wpb) {
-    int8_t *sigma_row = sigma + (int64_t)b * N;
-    __syncwarp();
-    for (int i = lane; i < N; i += 32) xs[i] = sigma_row[i];
-    __syncwarp();
-    int hop = 0;
-    for (int w = lane; w < nwords; w += 32) {
-      uint32_t bits = 0u;
-      for (int t = 0; t < 32; ++t) {
-        const int q = 32 * w + t;
-        if (q < C && xs[cl[2 * q]] != xs[cl[2 * q + 1]]) bits |= 1u << t;
-      }
-      mask[w] = bits;
-      hop += __popc(bits);
-    }
-    hop = warp_sum_int(hop);
-    __syncwarp();
-    float logpsi = 0.0f;
-    auto recompute = [&]() {
-      float part = 0.0f;
-      for (int j = lane; j < M; j += 32) {
-        float acc = __ldg(bg + j);
-        for (int i = 0; i < N; ++i) acc += (float)xs[i] * __ldg(Wg + (int64_t)i * M + j);
-        ths[j] = acc;
-        part += log_cosh_fast(acc);
-      }
-      for (int i = lane; i < N; i += 32) part += (float)xs[i] * __ldg(ag + i);
-      logpsi = warp_sum(part);
-      __syncwarp();
-    };
-    int64_t acc_count = 0;
-    const int total = n_discard + L;
-    for (int step = 0; step < total; ++step) {
-      recompute();
-      for (int p = 0; p < sweep; ++p) {
-        const uint64_t pidx = counter + (uint64_t)step * sweep + p;
-        u32x4 rr = philox4x32_10(u32x4{(uint32_t)pidx, (uint32_t)(pidx >> 32), (uint32_t)b, 0u},
-                                 k0, k1);
-        if (hop == 0) continue;  // no move possible: rejected
-        int k = (int)below(rr.x, (uint32_t)hop);
-        const uint32_t wbits = lane < nwords ? mask[lane] : 0u;
-        const int cnt = __popc(wbits);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        const int excl = incl - cnt;
-        const bool owner = excl <= k && k < incl;
-        const unsigned ob = __ballot_sync(0xffffffffu, owner);
-        if (ob == 0u) continue;  // unreachable while hop matches the mask
-        const int src = __ffs(ob) - 1;
-        int pick = -1;
-        if (owner) pick = 32 * lane + nth_set_bit(wbits, k - excl);
-        pick = __shfl_sync(0xffffffffu, pick, src);
-        if (pick < 0 || pick >= C) continue;  // likewise unreachable; never out of range
-        const int su = cl[2 * pick], sv = cl[2 * pick + 1];
-        const int8_t xu = xs[su], xv = xs[sv];
-        const float du = (float)(xv - xu), dv = (float)(xu - xv);
-        int q = -1, newh = 0;
-        int hop_new;
-        if (!full_recount) {
-          const int site = lane < 16 ? su : sv, slot = lane & 15;
-          if (slot < deg[site]) {
-            q = inc[site * XS_MAXDEG + slot];
-            const int a0 = cl[2 * q], a1 = cl[2 * q + 1];
-            if (lane >= 16 && (a0 == su || a1 == su)) q = -1;
-            if (q >= 0) {
-              const int8_t x0 = a0 == su ? xv : (a0 == sv ? xu : xs[a0]);
-              const int8_t x1 = a1 == su ? xv : (a1 == sv ? xu : xs[a1]);
-              newh = x0 != x1;
-            }
-          }
-          const int oldh = q >= 0 ? (int)((mask[q >> 5] >> (q & 31)) & 1u) : 0;
-          hop_new = hop + warp_sum_int(q >= 0 ? newh - oldh : 0);
-        } else {
-          int h2 = 0;
-          for (int q0 = 0; q0 < C; q0 += 32) {
-            const int qq = q0 + lane;
-            if (qq < C) {
-              const int a0 = cl[2 * qq], a1 = cl[2 * qq + 1];
-              const int8_t x0 = a0 == su ? xv : (a0 == sv ? xu : xs[a0]);
-              const int8_t x1 = a1 == su ? xv : (a1 == sv ? xu : xs[a1]);
-              h2 += x0 != x1;
-            }
-          }
-          hop_new = warp_sum_int(h2);
-        }
-        const float corr = logtab[hop] - logtab[hop_new];
-        float sacc = 0.0f;
-        const float *Wu = Wg + (int64_t)su * M, *Wv = Wg + (int64_t)sv * M;
-#pragma unroll 8
-        for (int j = lane; j < M; j += 32) {
-          const float th = ths[j];
-          float t = th + du * __ldg(Wu + j);
-          t += dv * __ldg(Wv + j);
-          sacc += log_cosh_fast(t) - log_cosh_fast(th);
-        }
-        float s = warp_sum(sacc);
-        s += du * __ldg(ag + su);
-        s += dv * __ldg(ag + sv);
-        const float dlp = 2.0f * s;
-        const float u = u01f(rr.y);
-        if (u < expf(dlp + corr)) {
-#pragma unroll 8
-          for (int j = lane; j < M; j += 32) {
-            float t = ths[j] + du * __ldg(Wu + j);
-            t += dv * __ldg(Wv + j);
-            ths[j] = t;
-          }
-          __syncwarp();
-          if (lane == 0) {
-            xs[su] = (int8_t)(xu + (int)du);
-            xs[sv] = (int8_t)(xv + (int)dv);
-          }
-          if (!full_recount) {
-            if (q >= 0) {
-              const uint32_t bit = 1u << (q & 31);
-              if (newh) atomicOr(&mask[q >> 5], bit);
-              else atomicAnd(&mask[q >> 5], ~bit);
-            }
-          } else {
-            __syncwarp();
-            for (int w = lane; w < nwords; w += 32) {
-              uint32_t bits = 0u;
-              for (int t = 0; t < 32; ++t) {
-                const int qq = 32 * w + t;
-                if (qq < C && xs[cl[2 * qq]] != xs[cl[2 * qq + 1]]) bits |= 1u << t;
-              }
-              mask[w] = bits;
-            }
-          }
-          hop = hop_new;
-          logpsi += s;
-          ++acc_count;
-        }
-        __syncwarp();
-      }
-      if (step >= n_discard) {
-        int8_t *dst = samples + ((int64_t)b * L + (step - n_discard)) * N;
-        for (int i = lane; i < N; i += 32) dst[i] = xs[i];
-      }
-    }
-    recompute();
-    for (int i = lane; i < N; i += 32) sigma_row[i] = xs[i];
-    if (lane == 0) {
-      log_prob[b] = 2.0 * (double)logpsi;
-      n_accepted[b] += acc_count;
-    }
-  }
-}
-
-static size_t exchange_l2_smem_bytes(int N, int M, int C, int wpb) {
-  const int nwords = (C + 31) >> 5;
-  size_t bytes = (size_t)(C + 1) * 4 + (size_t)C * 4 + (size_t)N * XS_MAXDEG * 2 + 4 +
-                 (size_t)N * 4 + 16;
-  bytes += (size_t)wpb * (4 * (size_t)M + (((size_t)N + 15) & ~size_t(15)) + 4 * (size_t)nwords);
-  return bytes + 64;
-}
-
-// Dynamic shared memory a block may use on this GPU (227 KB on sm_100 / sm_103),
-// less the kernel's static variable.
-constexpr size_t XL_SMEM_MAX = 227 * 1024 - 64;
-
-// Chains per block of the L2 kernel: as many as fit (at most XL_WARPS), 0 if
-// fewer than 4 do.
-static int exchange_l2_warps(int N, int M, int C) {
-  int w = XL_WARPS;
-  while (w >= 4 && exchange_l2_smem_bytes(N, M, C, w) > XL_SMEM_MAX) --w;
-  return w >= 4 ? w : 0;
-}
-
-static int launch_exchange_l2(cudaStream_t st, const float *p, int N, int M, int8_t *sigma,
-                              double *log_prob, int64_t *n_acc, int B, int sweep, int n_discard,
-                              int L, int8_t *samples, uint32_t k0, uint32_t k1, uint64_t counter,
-                              const int32_t *clusters, int C, int sms) {
-  const int wpb = exchange_l2_warps(N, M, C);
-  VMCK_REQUIRE(wpb >= 4, "exchange L2 kernel: M too large");
-  const size_t smem = exchange_l2_smem_bytes(N, M, C, wpb);
-  VMCK_CUDA(cudaFuncSetAttribute(metropolis_exchange_l2_kernel,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int grid = (int)std::min<int64_t>(((int64_t)B + wpb - 1) / wpb, sms);
-  metropolis_exchange_l2_kernel<<<grid, 32 * wpb, smem, st>>>(
-      p, N, M, sigma, log_prob, n_acc, B, sweep, n_discard, L, samples, k0, k1, counter, clusters,
-      C);
-  return check_launch("metropolis_sample (exchange, weights through L2)");
-}
-
 template <typename T>
 int launch_metropolis(cudaStream_t st, const void *params, int N, int M, int8_t *sigma,
                       double *log_prob, int64_t *n_acc, int B, int sweep, int n_discard, int L,
@@ -531,20 +266,12 @@ int launch_metropolis(cudaStream_t st, const void *params, int N, int M, int8_t 
   // call): the parity tests run both kernels on the same seeds.
   const char *generic = getenv("VMCK_EXCHANGE_GENERIC");
   const bool force_generic = generic && generic[0] == '1';
-  if (!force_generic && filtered_fits(rule, N, M, C)) {
-    const SweepArgs a{params,  N,       M,   sigma, log_prob, n_acc,    B, sweep, n_discard, L,
-                      samples, k0,      k1,  counter, clusters, C};
-    return launch_filtered(st, sizeof(T) == 8 ? VMCK_F64 : VMCK_F32, rule, a);
-  }
-  if (sizeof(T) == 4 && rule == 1 && C <= 1024 && M > 512 && !force_generic &&
-      exchange_l2_warps(N, M, C) > 0) {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return launch_exchange_l2(st, reinterpret_cast<const float *>(params), N, M, sigma, log_prob,
-                              n_acc, B, sweep, n_discard, L, samples, k0, k1, counter, clusters, C,
-                              sms);
-  }
+  const SweepArgs a{params,  N,       M,   sigma,   log_prob, n_acc,    B, sweep, n_discard, L,
+                    samples, k0,      k1,  counter, clusters, C};
+  constexpr int dtype = sizeof(T) == 8 ? VMCK_F64 : VMCK_F32;
+  if (!force_generic && filtered_fits(rule, N, M, C)) return launch_filtered(st, dtype, rule, a);
+  if (!force_generic && filtered_l2_fits(dtype, rule, N, M, C))
+    return launch_filtered_l2(st, dtype, rule, a);
   if (rule == 0) {
     if (smem > 48 * 1024)
       VMCK_CUDA(cudaFuncSetAttribute(metropolis_kernel<T, 0>,

@@ -35,26 +35,19 @@
 // 0.67 ms; FP64 Exchange, N = 36, M = 72, 1,024 chains 7.77 -> 0.52 ms; FP32
 // Exchange, 10 x 10 J1-J2, M = 400, 4,096 chains 3.45 -> 1.22 ms (about 880 warp
 // instructions per proposal before).
-#include "sampler_filter.cuh"
-
 #include <algorithm>
+
+#include "filter_common.cuh"
 
 namespace vmck {
 
 namespace {
 
 constexpr int FS_MAX_WARPS = 28;
-constexpr size_t FS_SMEM_MAX = 227 * 1024 - 256;
 
 template <typename T, int R>
 constexpr int max_warps() {  // by registers: theta, t (and the low parts)
   return sizeof(T) == 4 ? FS_MAX_WARPS : (R <= 8 ? 24 : 20);
-}
-
-__device__ __forceinline__ float ex2_fast(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 
 // Row layout of the shared weights: hidden unit l + 32 r at quad r / 4 of lane l
@@ -97,90 +90,7 @@ __host__ __device__ inline FilterSmem filter_smem(int rule, int N, int R, int C)
   return s;
 }
 
-// The plain kernel's decision in FP64, theta formed from scratch for the spins in
-// the words xb (word l in lane l).
-__device__ __noinline__ bool exact_accept_f64(const double *__restrict__ params, int N, int M,
-                                              uint32_t xb, int su, int sv, int du, int hop,
-                                              int hop_new, uint32_t ry, uint32_t rz) {
-  const int lane = threadIdx.x & 31;
-  const double *W = params + M, *a = params + M + (int64_t)N * M;
-  double s = 0.0;
-  for (int j0 = 0; j0 < M; j0 += 32) {
-    const int j = j0 + lane;
-    const bool in = j < M;
-    const double *Wj = W + (in ? j : 0);
-    double th = in ? params[j] : 0.0;
-    for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-      const int i1 = min(32, N - 32 * w);
-      for (int q = 0; q < i1; ++q) {
-        const double v = Wj[(int64_t)(32 * w + q) * M];
-        th += (bits >> q) & 1u ? v : -v;
-      }
-    }
-    if (in) {
-      double t = th + (double)du * Wj[(int64_t)su * M];
-      if (sv >= 0) t -= (double)du * Wj[(int64_t)sv * M];
-      s += log_cosh(t) - log_cosh(th);
-    }
-  }
-  s = warp_sum(s);
-  s += (double)du * a[su];
-  double corr = 0.0;
-  if (sv >= 0) {
-    s -= (double)du * a[sv];
-    corr = log((double)hop) - log((double)hop_new);
-  }
-  return u01d(ry, rz) < exp(2.0 * s + corr);
-}
-
-// log psi of the final state in FP64, in metropolis_kernel's order.
-__device__ __noinline__ double final_logpsi_f64(const double *__restrict__ params, int N, int M,
-                                                uint32_t xb) {
-  const int lane = threadIdx.x & 31;
-  const double *W = params + M, *a = params + M + (int64_t)N * M;
-  double part = 0.0;
-  for (int j0 = 0; j0 < M; j0 += 32) {
-    const int j = j0 + lane;
-    const bool in = j < M;
-    const double *Wj = W + (in ? j : 0);
-    double th = in ? params[j] : 0.0;
-    for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-      const int i1 = min(32, N - 32 * w);
-      for (int q = 0; q < i1; ++q) {
-        const double v = Wj[(int64_t)(32 * w + q) * M];
-        th += (bits >> q) & 1u ? v : -v;
-      }
-    }
-    if (in) part += log_cosh(th);
-  }
-  for (int w = 0; 32 * w < N; ++w) {
-    const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-    const int i = 32 * w + lane;
-    if (i < N) part += (bits >> lane) & 1u ? a[i] : -a[i];
-  }
-  return warp_sum(part);
-}
-
 }  // namespace
-
-// eps, the filter's margin on ln u - (2 s + corr).  Per hidden unit: ex2.approx
-// and lg2.approx are off by 2^-22 each, the product and the argument of the
-// exponential by 2^-24, in t and in theta (A_UNIT); FP32 only: the plain kernel's
-// log_cosh_fast by 5e-7 + 2^-23 |x| (B_UNIT, with its |x| part in the next term).
-// Per unit of S = sum |t| + |theta|: the roundings of theta + delta and of the
-// lane's R additions, 2^-24 each.  The lanes' sums go to the warp total as
-// integers in units of 2^-19 (FIXED: half a unit per lane).  FP32 only: the plain
-// kernel's summation rounds R + 6 times, each time by 2^-24 of at most
-// sum_j |t - theta| <= 2 (|W_u|_1 + |W_v|_1).  FP64 only: the FP32 weights are off
-// by 2^-24 of themselves, theta and t by 2^-24 of sum |W| + |b| each and delta by 2
-// more of it.  ln u:
-// lg2.approx (2^-22 of at most 32) and, in FP64, the 21 low bits of u, left out
-// (2^-16).  Each constant is at least 1.5 times the bound it stands for.
-constexpr float A_UNIT = 1.3e-6f, B_UNIT = 1.6e-6f, ROUND = 5.97e-8f, FIXED = 4.6e-5f,
-                LN_U = 4e-5f, X_REL = 1e-6f;
-constexpr float SUM_UNIT = 1.0f / 524288.0f, SUM_MAX = 126.0f;  // 32 * 126 * 2^19 < 2^31
 
 template <typename T, int RULE, int R>
 __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
@@ -208,29 +118,16 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
       Ws[i * (32 * R) + row_pos<R>(j)] = v;
     }
     for (int i = tid; i < N; i += blockDim.x) as[i] = (float)params[M + (int64_t)N * M + i];
-    if (RULE == 1) {
-      for (int k = tid; k <= C; k += blockDim.x) logtab[k] = logf((float)k);
-      for (int q = tid; q < C; q += blockDim.x)
-        cl[q] = (uint32_t)A.clusters[2 * q] | (uint32_t)A.clusters[2 * q + 1] << 16;
-      for (int e = tid; e < N * nwords; e += blockDim.x) inc[e] = 0u;
-    }
     if (tid == 0) all_l1 = 0.0f;
+    if (RULE == 1) stage_rule(A, nwords, logtab, cl, inc);
     __syncthreads();
-    if (RULE == 1) {
-      for (int q = tid; q < C; q += blockDim.x) {
-        const int u = (int)(cl[q] & 0xffffu), v = (int)(cl[q] >> 16);
-        if (u != v) {  // a cluster of one site twice is never hoppable
-          atomicOr(&inc[u * nwords + (q >> 5)], 1u << (q & 31));
-          atomicOr(&inc[v * nwords + (q >> 5)], 1u << (q & 31));
-        }
-      }
-    }
     for (int i = warp; i <= N; i += (int)(blockDim.x >> 5)) {
       float w[R], s = 0.0f;
       load_row<R>(Ws + i * (32 * R), lane, w);
 #pragma unroll
       for (int r = 0; r < R; ++r) s += fabsf(w[r]);
       s = warp_sum(s);
+      if (i < N) s += fabsf(as[i]);
       if (lane == 0) {
         if (i < N) l1[i] = s;
         atomicAdd(&all_l1, s);  // a bound: the order of the sum does not matter
@@ -240,45 +137,9 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
   }
   const int b = blockIdx.x * wpb + warp;
   if (warp >= wpb || b >= A.B) return;  // the other warps only helped staging
-  // spins: bit i of word l (lane l) set where x = +1
-  uint32_t xb = 0u;
-  {
-    const int8_t *row = A.sigma + (int64_t)b * N;
-    for (int w = 0; 32 * w < N; ++w) {
-      const int i = 32 * w + lane;
-      const uint32_t m = __ballot_sync(0xffffffffu, i < N && row[i] > 0);
-      if (lane == w) xb = m;
-    }
-  }
-  auto spin_up = [&](int i) -> bool {
-    return (__shfl_sync(0xffffffffu, xb, i >> 5) >> (i & 31)) & 1u;
-  };
-  // hoppable clusters: bit q of word l, their count and the counts before word l
-  uint32_t hb = 0u;
-  int hop = 0, before = 0, cnt = 0;
-  auto prefix = [&]() {
-    cnt = __popc(hb);
-    int inclusive = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inclusive, o);
-      if (lane >= o) inclusive += v;
-    }
-    before = inclusive - cnt;
-  };
-  if (RULE == 1) {
-    for (int w = 0; w < nwords; ++w) {
-      const int q = 32 * w + lane;
-      const uint32_t c = q < C ? cl[q] : 0u;
-      const int u = (int)(c & 0xffffu), v = (int)(c >> 16);
-      const uint32_t xu = __shfl_sync(0xffffffffu, xb, u >> 5) >> (u & 31);
-      const uint32_t xv = __shfl_sync(0xffffffffu, xb, v >> 5) >> (v & 31);
-      const uint32_t m = __ballot_sync(0xffffffffu, q < C && ((xu ^ xv) & 1u));
-      if (lane == w) hb = m;
-    }
-    prefix();
-    hop = __reduce_add_sync(0xffffffffu, cnt);
-  }
+  const RuleTables tables{logtab, cl, inc, C, nwords};
+  ChainBits<RULE> ch;
+  ch.load(A.sigma + (int64_t)b * N, N, tables);
 
   float th[R], lo[F64 ? R : 1];
   float sum_abs = 0.0f, log_prod = 0.0f;  // this lane's sum |theta|, lg2 prod (1 + e)
@@ -301,7 +162,7 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
       for (int r = 0; r < R; ++r) lo[r] = 0.0f;
     }
     for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
+      const uint32_t bits = __shfl_sync(0xffffffffu, ch.xb, w);
       const int i1 = min(32, N - 32 * w);
       for (int q = 0; q < i1; ++q) {
         const float x = (bits >> q) & 1u ? 1.0f : -1.0f;
@@ -339,49 +200,14 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
   int64_t acc_count = 0;
   for (int step = 0; step < total; ++step) {
     if (!F64) recompute();
-    uint32_t rx = 0, ry = 0, rz = 0;
-    float ln_u = 0.0f;
+    RandomWords<F64> rnd;
     for (int p = 0; p < A.sweep; ++p) {
-      if ((p & 31) == 0) {  // the random words of the next 32 proposals, one per lane
-        const uint64_t idx = A.counter + (uint64_t)step * A.sweep + p + lane;
-        const u32x4 r = philox4x32_10(
-            u32x4{(uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)b, 0u}, A.k0, A.k1);
-        rx = r.x;
-        ry = r.y;
-        rz = r.z;
-        // NaN (no decision by the filter) where the logarithm says too little
-        if (F64)
-          ln_u = ry >= 65536u ? (__log2f((float)ry) - 32.0f) * 0.693147181f : __int_as_float(-1);
-        else
-          ln_u = (ry >> 8) ? __logf(u01f(ry)) : __int_as_float(-1);
-      }
-      const uint32_t word = __shfl_sync(0xffffffffu, rx, p & 31);
-      int su, sv = -1, hop_new = 0;
-      uint32_t flip = 0u;
-      float corr = 0.0f;
-      if (RULE == 0) {
-        su = (int)below(word, (uint32_t)N);
-      } else {
-        if (hop == 0) continue;  // no move possible: rejected
-        // the k-th hoppable cluster: its word, then its bit
-        const int k = (int)below(word, (uint32_t)hop);
-        const unsigned own = __ballot_sync(0xffffffffu, before <= k && k < before + cnt);
-        if (own == 0u) continue;  // unreachable while the counts match the words
-        const int src = __ffs(own) - 1;
-        const uint32_t hw = __shfl_sync(0xffffffffu, hb, src);
-        const int nth = k - __shfl_sync(0xffffffffu, before, src);
-        const unsigned at = __ballot_sync(
-            0xffffffffu, ((hw >> lane) & 1u) && __popc(hw & ((1u << lane) - 1u)) == nth);
-        const int pick = 32 * src + __ffs(at) - 1;
-        if (pick >= C || at == 0u) continue;  // likewise; never index out of range
-        const uint32_t c = cl[pick];
-        su = (int)(c & 0xffffu);
-        sv = (int)(c >> 16);
-        if (lane < nwords) flip = inc[su * nwords + lane] ^ inc[sv * nwords + lane];
-        hop_new = hop + __reduce_add_sync(0xffffffffu, __popc(flip) - 2 * __popc(flip & hb));
-        corr = logtab[hop] - logtab[hop_new];
-      }
-      const int du = spin_up(su) ? -2 : 2;  // an Exchange partner changes by -du
+      if ((p & 31) == 0) rnd.draw(A, A.counter + (uint64_t)step * A.sweep + p, b);
+      Proposal pr;
+      if (!ch.propose(__shfl_sync(0xffffffffu, rnd.x, p & 31), N, tables, pr)) continue;
+      const int su = pr.su, sv = pr.sv;
+      const float corr = pr.corr;
+      const int du = ch.up(su) ? -2 : 2;  // an Exchange partner changes by -du
       const float fu = (float)du;
       float t[R];
       {
@@ -408,14 +234,15 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
       const float x = 2.0f * s + corr;
       float eps = eps0 + eps_s * (float)size + X_REL * (fabsf(x) + fabsf(corr));
       if (!F64) eps += eps_d * (RULE == 1 ? l1[su] + l1[sv] : l1[su]);
-      const float margin = __shfl_sync(0xffffffffu, ln_u, p & 31) - x;
+      const float margin = __shfl_sync(0xffffffffu, rnd.ln_u, p & 31) - x;
       bool accept = margin < 0.0f;
       if (!(fabsf(margin) > eps) || __any_sync(0xffffffffu, far)) {
         // too close to call: the plain kernel's own evaluation
         if constexpr (F64) {
-          accept = exact_accept_f64(static_cast<const double *>(A.params), N, M, xb, su, sv, du,
-                                    hop, hop_new, __shfl_sync(0xffffffffu, ry, p & 31),
-                                    __shfl_sync(0xffffffffu, rz, p & 31));
+          accept = exact_accept_f64(static_cast<const double *>(A.params), N, M, ch.xb, su,
+                                    sv, du, ch.hop, pr.hop_new,
+                                    __shfl_sync(0xffffffffu, rnd.y, p & 31),
+                                    __shfl_sync(0xffffffffu, rnd.z, p & 31));
         } else {
           float e = 0.0f;
 #pragma unroll
@@ -425,7 +252,7 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
           e += fu * as[su];
           if (RULE == 1) e += -fu * as[sv];
           const float dlp = 2.0f * e;
-          accept = u01f(__shfl_sync(0xffffffffu, ry, p & 31)) < expf(dlp + corr);
+          accept = u01f(__shfl_sync(0xffffffffu, rnd.y, p & 31)) < expf(dlp + corr);
         }
       }
       if (accept) {
@@ -459,27 +286,16 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
         }
         sum_abs = new_abs;
         log_prod = new_prod;
-        if (lane == (su >> 5)) xb ^= 1u << (su & 31);
-        if (RULE == 1) {
-          if (lane == (sv >> 5)) xb ^= 1u << (sv & 31);
-          hb ^= flip;
-          prefix();
-          hop = hop_new;
-        }
+        ch.apply(pr);
         ++acc_count;
       }
     }
-    if (step >= A.n_discard) {
-      int8_t *dst = A.samples + ((int64_t)b * A.L + (step - A.n_discard)) * N;
-      for (int w = 0; 32 * w < N; ++w) {
-        const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-        if (32 * w + lane < N) dst[32 * w + lane] = (bits >> lane) & 1u ? 1 : -1;
-      }
-    }
+    if (step >= A.n_discard)
+      ch.store(A.samples + ((int64_t)b * A.L + (step - A.n_discard)) * N, N);
   }
   T logpsi;
   if constexpr (F64) {
-    logpsi = final_logpsi_f64(static_cast<const double *>(A.params), N, M, xb);
+    logpsi = final_logpsi_f64(static_cast<const double *>(A.params), N, M, ch.xb);
   } else {
     recompute();
     float part = 0.0f;
@@ -487,19 +303,13 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
     for (int r = 0; r < R; ++r)
       if (lane + 32 * r < M) part += log_cosh_fast(th[r]);
     for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
+      const uint32_t bits = __shfl_sync(0xffffffffu, ch.xb, w);
       const int i = 32 * w + lane;
       if (i < N) part += ((bits >> lane) & 1u ? 1.0f : -1.0f) * as[i];
     }
     logpsi = warp_sum(part);
   }
-  {
-    int8_t *row = A.sigma + (int64_t)b * N;
-    for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-      if (32 * w + lane < N) row[32 * w + lane] = (bits >> lane) & 1u ? 1 : -1;
-    }
-  }
+  ch.store(A.sigma + (int64_t)b * N, N);
   if (lane == 0) {
     A.log_prob[b] = 2.0 * (double)logpsi;
     A.n_accepted[b] += acc_count;

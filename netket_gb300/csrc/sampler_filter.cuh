@@ -23,5 +23,8 @@ struct SweepArgs {
 // Whether the weights-in-shared-memory kernel takes this problem.
 bool filtered_fits(int rule, int N, int M, int C);
 int launch_filtered(cudaStream_t st, int dtype, int rule, const SweepArgs &a);
+// The same with the weights read through L2.
+bool filtered_l2_fits(int dtype, int rule, int N, int M, int C);
+int launch_filtered_l2(cudaStream_t st, int dtype, int rule, const SweepArgs &a);
 
 }  // namespace vmck

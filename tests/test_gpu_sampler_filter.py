@@ -83,3 +83,24 @@ def test_exchange_repeated_clusters(monkeypatch, dtype):
     cl = [(0, 1), (1, 0), (0, 1), (2, 2), (2, 3), (3, 4), (4, 5), (5, 6), (6, 7), (7, 0), (1, 2)]
     _both(monkeypatch, lambda: nk.sampler.MetropolisExchange(hi, clusters=cl, n_chains=33), model,
           flat)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("N,M,rule,chains,std", [
+    (200, 250, 0, 5, 0.05), (200, 256, 1, 3, 0.01), (140, 512, 0, 37, 0.3), (120, 513, 1, 37, 0.01),
+    (16, 1024, 1, 300, 0.3), (24, 1027, 0, 19, 0.01), (24, 2048, 1, 37, 0.1)])
+def test_weights_through_l2(monkeypatch, dtype, N, M, rule, chains, std):
+    """Weights too large for shared memory: the edges of the register forms (M =
+    256, 512, 1024, 2048 and beyond), rows that are not 16-byte aligned, fewer and
+    more chains than a block holds."""
+    import netket_gb300 as nk
+    model, flat = _model(nk, N, M, std, dtype)
+    if rule == 0:
+        hi = nk.hilbert.Spin(0.5, N)
+        make = lambda: nk.sampler.MetropolisLocal(hi, n_chains=chains, sweep_size=40)
+    else:
+        hi = nk.hilbert.Spin(0.5, N, total_sz=0)
+        g = nk.graph.Chain(N, max_neighbor_order=2)
+        make = lambda: nk.sampler.MetropolisExchange(hi, graph=g, d_max=2, n_chains=chains,
+                                                     sweep_size=40)
+    _both(monkeypatch, make, model, flat)
