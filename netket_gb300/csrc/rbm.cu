@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "eloc_f32.cuh"
 #include "localop.cuh"
 #include "pauli.cuh"
 #include "signsum.cuh"
@@ -704,6 +705,9 @@ extern "C" int vmck_rbm_eloc_ising(vmck_stream s, int32_t dtype, const void *par
   if (dtype == VMCK_F64)
     return launch_eloc_ising<double>(as_stream(s), params, N, M, x, n, edges, n_edges, h, J,
                                      eloc, logpsi_out);
+  if (dtype == VMCK_F32 && !logpsi_out && eloc_f32_takes(N, M, nullptr))
+    return eloc_f32_ising(as_stream(s), static_cast<const float *>(params), N, M, x, n, edges,
+                          n_edges, h, J, eloc);
   if (dtype == VMCK_F32)
     return launch_eloc_ising<float>(as_stream(s), params, N, M, x, n, edges, n_edges, h, J, eloc,
                                     logpsi_out);
@@ -721,6 +725,8 @@ extern "C" int vmck_rbm_eloc_local(vmck_stream s, int32_t dtype, const void *par
   if (n == 0) return VMCK_OK;
   if (dtype == VMCK_F64)
     return launch_eloc_local<double>(as_stream(s), params, N, M, x, n, *op, eloc, logpsi_out);
+  if (dtype == VMCK_F32 && !logpsi_out && eloc_f32_takes(N, M, op))
+    return eloc_f32_local(as_stream(s), static_cast<const float *>(params), N, M, x, n, *op, eloc);
   if (dtype == VMCK_F32)
     return launch_eloc_local<float>(as_stream(s), params, N, M, x, n, *op, eloc, logpsi_out);
   set_last_error("rbm_eloc_local: dtype %d unsupported", dtype);
