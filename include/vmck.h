@@ -424,6 +424,10 @@ int vmck_rbm_jacobian(vmck_stream s, int32_t dtype, const void *tanh_theta,
  * definite) with no cancellation against the mean.  status (nullable device int32) receives
  * VMCK_DEV_TIMEOUT if a tensor-core CTA's bounded wait ran out. */
 int64_t vmck_gram_workspace_size(int32_t N, int32_t M, int64_t n);
+/* Mode 0 with a workspace of at least this many doubles contracts on the tensor
+ * cores where that is faster: |t| <= 1 rounded to a multiple of 2^-55, in base-128
+ * digits whose products sum exactly (an error below an FP64 sum's). */
+int64_t vmck_gram_f64_workspace_size(int32_t N, int32_t M, int64_t n);
 
 int vmck_rbm_gram(vmck_ctx *ctx, vmck_stream s, int32_t mode, int32_t dtype,
                   const void *tanh_theta, const int8_t *x, int32_t N, int32_t M,

@@ -121,6 +121,7 @@ _SIGNATURES = {
     "vmck_rbm_jacobian": ([c_vp, c_i32, c_vp, c_vp, c_i32, c_i32, c_i64, c_vp, c_dbl, c_i32,
                            c_vp], c_i32),
     "vmck_gram_workspace_size": ([c_i32, c_i32, c_i64], c_i64),
+    "vmck_gram_f64_workspace_size": ([c_i32, c_i32, c_i64], c_i64),
     "vmck_rbm_gram": ([c_vp, c_vp, c_i32, c_i32, c_vp, c_vp, c_i32, c_i32, c_i64, c_vp, c_dbl,
                        c_vp, c_vp, c_vp, c_i64, c_vp], c_i32),
     "vmck_gram_dense": ([c_vp, c_vp, c_i32, c_vp, c_i64, c_i64, c_i32, c_dbl, c_vp], c_i32),

@@ -271,7 +271,9 @@ __global__ void __launch_bounds__(256) gram_simt_kernel(
     const T *__restrict__ t, const uint32_t *__restrict__ bits, int words, int N, int M, int64_t n,
     const double *__restrict__ g, const double *__restrict__ cptr, const float2 *__restrict__ hdf,
     const float2 *__restrict__ wdf, const float2 *__restrict__ s0sq_p, double inv_n,
-    double diag_shift, double *__restrict__ T64, float *__restrict__ T32) {
+    double diag_shift, double *__restrict__ T64, float *__restrict__ T32,
+    const int *__restrict__ only_if) {
+  if (only_if && *only_if == 0) return;  // the tensor-core form has written T
   __shared__ T ta[GK][GT];
   __shared__ T tb[GK][GT];
   __shared__ uint32_t ba[GT][9];
@@ -391,6 +393,10 @@ extern "C" int64_t vmck_gram_workspace_size(int32_t N, int32_t M, int64_t n) {
          2 + std::max(vmck::gram_tc_workspace_doubles(M, n), split) + 8;
 }
 
+extern "C" int64_t vmck_gram_f64_workspace_size(int32_t N, int32_t M, int64_t n) {
+  return vmck_gram_workspace_size(N, M, n) + vmck::gram64_tc_workspace_doubles(M, n);
+}
+
 extern "C" int vmck_rbm_gram(vmck_ctx *ctx, vmck_stream s, int32_t mode, int32_t dtype,
                              const void *tanh_theta, const int8_t *x, int32_t N, int32_t M,
                              int64_t n, const double *obar, double diag_shift, double *T64,
@@ -462,13 +468,22 @@ extern "C" int vmck_rbm_gram(vmck_ctx *ctx, vmck_stream s, int32_t mode, int32_t
   const int64_t nt = (n + GT - 1) / GT;
   const int64_t tiles = nt * (nt + 1) / 2;
   VMCK_REQUIRE(tiles < (1ll << 31), "too many tiles");
-  if (dtype == VMCK_F64)
+  if (dtype == VMCK_F64) {
+    const int *out_of_range = nullptr;
+    const int64_t base = vmck_gram_workspace_size(N, M, n);
+    if (gram64_tc_takes(M, n) &&
+        workspace_len >= base + gram64_tc_workspace_doubles(M, n)) {
+      if ((rc = gram64_tc_launch(st, static_cast<const double *>(tanh_theta), w.bits, words, N, M,
+                                 n, w.g, w.cptr, inv_n, diag_shift, T64, T32, workspace + base,
+                                 status, &out_of_range)))
+        return rc;
+    }
     gram_simt_kernel<double><<<(unsigned)tiles, 256, 0, st>>>(
         static_cast<const double *>(tanh_theta), w.bits, words, N, M, n, w.g, w.cptr, w.hdf,
-        w.wdf, w.s0sq, inv_n, diag_shift, T64, T32);
-  else
+        w.wdf, w.s0sq, inv_n, diag_shift, T64, T32, out_of_range);
+  } else
     gram_simt_kernel<float><<<(unsigned)tiles, 256, 0, st>>>(
         w.c, w.bits, words, N, M, n, w.g, w.cptr, w.hdf, w.wdf, w.s0sq, inv_n, diag_shift, T64,
-        T32);
+        T32, nullptr);
   return check_launch("gram simt");
 }

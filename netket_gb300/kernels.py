@@ -189,14 +189,16 @@ def jacobian_dense(tanh_t, x, N, M, col_mean, scale, out_dtype):
 
 def gram_structured(tanh_t, x, N, M, obar, diag_shift, mode, want_f32=False, status=None):
     """Lower triangle of T = O_L O_L^T + diag_shift I (n, n) FP64 (+ FP32 copy).
-    mode 0: FP64 CUDA cores; 1: FP32 CUDA cores; 2: tcgen05 BF16 hi/lo split;
+    mode 0: FP64 (exact integer products of base-128 digits on tcgen05 for large n n M,
+    else CUDA cores); 1: FP32 CUDA cores; 2: tcgen05 BF16 hi/lo split;
     3: tcgen05 single BF16; 4: tcgen05 FP16 hi/lo split (four products) with per-slab drained
     accumulation (the blocked-Cholesky GEMM) and a double-float assembly pass."""
     n = x.shape[0]
     T64 = torch.empty((n, n), dtype=torch.float64, device=x.device)
     T32 = torch.empty((n, n), dtype=torch.float32, device=x.device) if want_f32 else None
-    ws = torch.empty(nat.lib().vmck_gram_workspace_size(N, M, n), dtype=torch.float64,
-                     device=x.device)
+    size = (nat.lib().vmck_gram_f64_workspace_size if int(mode) == 0
+            else nat.lib().vmck_gram_workspace_size)
+    ws = torch.empty(size(N, M, n), dtype=torch.float64, device=x.device)
     nat.check(nat.lib().vmck_rbm_gram(nat.ctx(), nat.stream(), int(mode),
                                       nat.dtype_code(tanh_t.dtype), nat.ptr(tanh_t), nat.ptr(x), N,
                                       M, n, nat.ptr(obar), float(diag_shift), nat.ptr(T64),
