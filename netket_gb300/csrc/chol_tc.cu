@@ -111,17 +111,26 @@ __global__ void chol_split_rows_kernel(const float *__restrict__ A, int64_t n, i
 // from the old C values, loaded while the tile's first slab runs, so the
 // write-out only stores.  Waits for work are bounded by the library's wait limit; a wait that
 // runs out sets VMCK_DEV_TIMEOUT and the CTA winds down.
-constexpr int G_BM = 128, G_BN = 256, G_BK = 64, G_STAGES = 2;
-constexpr int G_EPI_WARPS = 16;  // four per tensor-memory lane quarter, 64 columns each
+//
+// BN = 256 columns per tile; one-row-tile launches (the factorisation's chain, which
+// waits for them) take 128 or 64 where the columns then still fit one wave: the
+// write-out of a tile (4 + 4 bytes per entry, one SM's stores) is most of such a
+// launch, so it shrinks with the tile.  Panel row and next rows at n = 4,096, K =
+// 128: 13 and 14 us -> 5 and 7 us (with the split copy stored two rows at a time).
+constexpr int G_BM = 128, G_BK = 64, G_STAGES = 2;
+constexpr int G_EPI_WARPS = 16;  // four per tensor-memory lane quarter, BN / 4 columns each
 constexpr int G_THREADS = 32 * (2 + G_EPI_WARPS);
-constexpr int G_TMEM_COLS = 2 * G_BN;  // D1 (hi * hi, one slab), D2 (cross terms, one tile)
-constexpr int G_COLS = G_BN / 4;       // columns per epilogue warp
 constexpr int G_A_BYTES = G_BM * G_BK * 2;  // 16 KB (one of hi / lo)
-constexpr int G_B_BYTES = G_BN * G_BK * 2;  // 32 KB
-constexpr int G_STAGE_BYTES = 2 * G_A_BYTES + 2 * G_B_BYTES;
 constexpr int G_UMMA_K = 16;
 constexpr int G_CHUNK = 8;  // epilogue columns per tensor-memory load
-constexpr int G_NCH = G_COLS / G_CHUNK;
+template <int BN>
+struct GemmTile {
+  static constexpr int TMEM_COLS = 2 * BN;  // D1 (hi * hi, one slab), D2 (cross terms, one tile)
+  static constexpr int COLS = BN / 4;       // columns per epilogue warp
+  static constexpr int B_BYTES = BN * G_BK * 2;
+  static constexpr int STAGE_BYTES = 2 * G_A_BYTES + 2 * B_BYTES;
+  static constexpr int BOX = BN < G_BM ? BN : G_BM;  // rows of a B operand copy
+};
 
 struct GemmParams {
   int M, N, K;
@@ -147,12 +156,18 @@ struct GemmParams {
 };
 
 // Tile t -> (mi, ni).  Upper-triangular launches (BN = 2 BM, common origin):
-// column tile ni holds row tiles 0 .. min(mt, 2 ni + 2) - 1.
+// column tile ni holds row tiles 0 .. min(mt, 2 ni + 2) - 1.  With one row tile
+// (any BN) tile t is column tile t.
 __device__ __forceinline__ int64_t tri_cum(int64_t ni, int64_t mt) {
   const int64_t h = mt / 2;
   return ni <= h ? ni * (ni + 1) : h * (h + 1) + (ni - h) * mt;
 }
 __device__ __forceinline__ void gemm_tile(const GemmParams &g, int64_t t, int &mi, int &ni) {
+  if (g.mt == 1) {
+    mi = 0;
+    ni = (int)t;
+    return;
+  }
   if (!g.tri) {
     mi = (int)(t % g.mt);
     ni = (int)(t / g.mt);
@@ -187,10 +202,14 @@ __device__ __forceinline__ void gemm_work(const GemmParams &g, int64_t t, int &m
   C = g.C + z * g.zstride;
 }
 
+template <int BN>
 __global__ void __launch_bounds__(G_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
                    const __grid_constant__ CUtensorMap mBh, const __grid_constant__ CUtensorMap mBl,
                    GemmParams g) {
+  constexpr int G_BN = BN, G_TMEM_COLS = GemmTile<BN>::TMEM_COLS, G_COLS = GemmTile<BN>::COLS;
+  constexpr int G_B_BYTES = GemmTile<BN>::B_BYTES, G_STAGE_BYTES = GemmTile<BN>::STAGE_BYTES;
+  constexpr int G_NCH = G_COLS / G_CHUNK;
   extern __shared__ __align__(1024) unsigned char g_smem_raw[];
   unsigned char *smem = reinterpret_cast<unsigned char *>(
       (reinterpret_cast<uintptr_t>(g_smem_raw) + 1023) & ~uintptr_t(1023));
@@ -269,11 +288,12 @@ __global__ void __launch_bounds__(G_THREADS, 1)
           mbar_expect_tx(&full[s], G_STAGE_BYTES);
           tma_load_2d(st, &mAh, &full[s], x, ya);
           tma_load_2d(st + G_A_BYTES, &mAl, &full[s], x, ya);
-          tma_load_2d(st + 2 * G_A_BYTES, &mBh, &full[s], x, yb);
-          tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES / 2, &mBh, &full[s], x, yb + G_BN / 2);
-          tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES, &mBl, &full[s], x, yb);
-          tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES + G_B_BYTES / 2, &mBl, &full[s], x,
-                      yb + G_BN / 2);
+          constexpr int BOX = GemmTile<BN>::BOX;
+#pragma unroll
+          for (int r = 0; r < G_BN; r += BOX) {
+            tma_load_2d(st + 2 * G_A_BYTES + r * G_BK * 2, &mBh, &full[s], x, yb + r);
+            tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES + r * G_BK * 2, &mBl, &full[s], x, yb + r);
+          }
         }
       }
       // every copy issued must land before the CTA may exit
@@ -416,24 +436,39 @@ __global__ void __launch_bounds__(G_THREADS, 1)
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(d2_empty);
-      // write-out (stores only)
+      // write-out (stores only).  The split copy goes out two rows at a time: lane
+      // pairs exchange one column each, so an even lane stores rows m, m + 1 of the
+      // even column and an odd lane rows m - 1, m of the odd one
       float *cp = Crow + (int64_t)nbase * g.ldc;
-      const bool split_row = g.oh && row_ok && m < g.o_rows;
+      const bool odd = lane & 1;
 #pragma unroll
-      for (int i = 0; i < G_COLS; ++i) {
+      for (int i = 0; i < G_COLS; i += 2) {
         const int nn = nbase + i;
-        if (row_ok && nn < g.N && (!g.tri || m <= nn)) {
-          const float val = alpha * acc[i];
-          *cp = val;
-          if (split_row && nn >= g.o_col0) {
-            __half hi, lo;
-            split_f16(val, so, hi, lo);
-            const int64_t o = (int64_t)(nn - g.o_col0) * g.ldo + m;
-            g.oh[o] = hi;
-            g.ol[o] = lo;
+        const float v0 = alpha * acc[i], v1 = alpha * acc[i + 1];
+        if (row_ok && nn < g.N && (!g.tri || m <= nn)) *cp = v0;
+        if (row_ok && nn + 1 < g.N && (!g.tri || m <= nn + 1)) cp[g.ldc] = v1;
+        cp += 2 * g.ldc;
+        if (g.oh && nn + 1 >= g.o_col0) {  // warp-uniform
+          __half h0, l0, h1, l1;
+          split_f16(v0, so, h0, l0);
+          split_f16(v1, so, h1, l1);
+          const __half2 mine = odd ? __halves2half2(h1, l1) : __halves2half2(h0, l0);
+          const __half2 give = odd ? __halves2half2(h0, l0) : __halves2half2(h1, l1);
+          const __half2 got = __shfl_xor_sync(0xffffffffu, give, 1);
+          const __half2 first = odd ? got : mine, second = odd ? mine : got;  // rows in order
+          const int c = nn + (odd ? 1 : 0), m0 = m & ~1;
+          const int rows = min(g.o_rows, g.tri ? min(g.M, c + 1) : g.M);
+          if (c < g.N && c >= g.o_col0 && m0 < rows) {
+            const int64_t o = (int64_t)(c - g.o_col0) * g.ldo + m0;
+            if (m0 + 1 < rows) {
+              *reinterpret_cast<__half2 *>(g.oh + o) = __lows2half2(first, second);
+              *reinterpret_cast<__half2 *>(g.ol + o) = __highs2half2(first, second);
+            } else {
+              g.oh[o] = __low2half(first);
+              g.ol[o] = __high2half(first);
+            }
           }
         }
-        cp += g.ldc;
       }
     }
   }
@@ -449,26 +484,245 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 
 // ------------------------------------------------------------ the leaf
 // One CTA factors the mp x mp (mp <= 128) diagonal block at (r0, r0) of the
-// column-major upper A in shared memory and forms X = U^-1.  Per 32-wide
-// sub-panel p:
+// column-major upper A in shared memory, A = U^T U, and forms X = U^-1.  Per 32-row
+// panel p:
 //   (a) warp 0 factors the 32 x 32 diagonal block, lane l holding column l in
-//       registers: per pivot one shuffle and one FMA per row, the rows shifted
-//       down one register per step so the step loop has a single compact body
-//       (entries below the diagonal are updated too and never read);
-//   (b) the panel row U_pp^-T A_p,j by forward substitution, two threads per
-//       column j (even / odd rows), fully unrolled;
-//   (c) the rank-32 update of the trailing block in 4 x 4 register tiles.
-// Then warps 0-3 invert the four 32 x 32 diagonal blocks and all threads form
-// the off-diagonal blocks of X by block back substitution, four outputs per
-// thread at a time.
+//       registers, four pivots at a time: every lane factors the 4 x 4 pivot block
+//       from a shared-memory broadcast (no shuffle in the pivot chain) and solves its
+//       own four entries, and the rows below get one rank-4 update with a row's four
+//       multipliers in one 16-byte broadcast.  The next four rows are updated first,
+//       so their pivot chain overlaps the update of the others; the rows shift down
+//       four registers per step, so the step loop has one compact body;
+//   (b) the panel row U_pp^-T A_p,j by forward substitution, one thread per column;
+//   (c) the rank-32 update of the trailing block in 4 x 4 register tiles: the next
+//       diagonal block first, so that warp 0 goes on to its (a) while the other
+//       warps update the rest;
+//   (d) meanwhile warp 7 inverts U_pp (lane l solves U x = e_l from the bottom row
+//       up).
+// The off-diagonal blocks X_IJ = -X_II sum_K U_IK X_KJ follow as far as they can
+// behind the last factor and inversion, then the last block column, four warps a
+// block (one warp issues an FMA every 1.75 clocks; with eight warps the operands'
+// shared-memory reads bound it).
+// Every entry takes the same operations in the same order as a right-looking
+// elimination one pivot at a time would give it.
 // Writes U in place, X split into K-contiguous rows (xh/xl[m * 128 + k] = X(k, m),
 // scale from max |X| into *scale_x) and Y = X^T zero-padded column-major
 // 128 x 128 (the refinement's triangular solves).  Rows / columns past mp are
 // the identity.  A non-positive or NaN pivot raises VMCK_DEV_NOT_SPD and is
 // replaced by 1.
-constexpr int LB = 128, LLD = LB + 1, LEAF_T = 256;
-constexpr int LPAD = 64;  // zeros after S: the diagonal inverse reads up to 31 floats past it
-constexpr size_t CHOL_LEAF_SMEM = (size_t)(2 * LB * LLD + LPAD + LB + 3 * 32 * 33) * sizeof(float);
+//
+// One SM is busy and 128 of these are in a row at n = 16,384, so only its latency
+// counts: 62,000 clocks, 33 us (50 us with one pivot at a time in one warp and each
+// phase after the other; of these now: load 4, factors 23, panel rows and updates 9,
+// X 16, outputs 9 thousand).
+constexpr int LB = 128, LLD = LB + 4, LEAF_T = 256;
+constexpr int LRD = 36;  // row stride of a diagonal block's shifted rows
+constexpr size_t CHOL_LEAF_SMEM =
+    (size_t)(2 * LB * LLD + 2 * 32 * LRD + 3 * 32 * LRD + LB + 4 * 32 + 4 * 64) * sizeof(float);
+
+// All threads, or the seven warps that factor.
+__device__ __forceinline__ void leaf_sync_all() { __syncthreads(); }
+__device__ __forceinline__ void leaf_sync_main() {
+  asm volatile("bar.sync 1, 224;" ::: "memory");
+}
+
+// The 4 x 4 pivot block (columns a0 .. a3, upper part) of the four rows c: the lane's
+// own entries of U in v, the inverse roots in inv.
+struct LeafPivots {
+  float v[4], inv[4];
+  int bad;  // bit m: pivot m was not positive and is replaced by 1
+};
+__device__ __forceinline__ LeafPivots leaf_pivots(const float4 &a0, const float4 &a1,
+                                                  const float4 &a2, const float4 &a3,
+                                                  const float (&c)[4]) {
+  LeafPivots p;
+  p.bad = 0;
+  auto root = [&](float d, int m) {
+    if (!(d > 0.0f)) {
+      p.bad |= 1 << m;
+      d = 1.0f;
+    }
+    return rsqrtf(d);
+  };
+  const float i0 = root(a0.x, 0);
+  const float u01 = a1.x * i0, u02 = a2.x * i0, u03 = a3.x * i0;
+  const float i1 = root(fmaf(-u01, u01, a1.y), 1);
+  const float u12 = fmaf(-u01, u02, a2.y) * i1, u13 = fmaf(-u01, u03, a3.y) * i1;
+  const float i2 = root(fmaf(-u12, u12, fmaf(-u02, u02, a2.z)), 2);
+  const float u23 = fmaf(-u12, u13, fmaf(-u02, u03, a3.z)) * i2;
+  const float i3 = root(fmaf(-u23, u23, fmaf(-u13, u13, fmaf(-u03, u03, a3.w))), 3);
+  p.v[0] = c[0] * i0;
+  p.v[1] = fmaf(-u01, p.v[0], c[1]) * i1;
+  p.v[2] = fmaf(-u12, p.v[1], fmaf(-u02, p.v[0], c[2])) * i2;
+  p.v[3] = fmaf(-u23, p.v[2], fmaf(-u13, p.v[1], fmaf(-u03, p.v[0], c[3]))) * i3;
+  p.inv[0] = i0;
+  p.inv[1] = i1;
+  p.inv[2] = i2;
+  p.inv[3] = i3;
+  return p;
+}
+
+// (a): U_pp into S, its rows shifted left of their diagonal into shifted[k][q] =
+// U(k, k + 1 + q) (zero past the block), 1 / U(k, k) into rd.  Returns whether a
+// pivot was replaced.
+__device__ __forceinline__ bool leaf_factor32(float *S, int P, float *shifted, float *rd,
+                                              float *piv, float *mul) {
+  const int lane = threadIdx.x & 31;
+  // at step k0, c[i] holds row k0 + i of column P + lane
+  float c[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) c[i] = S[(P + i) * LLD + P + lane];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) shifted[i * LRD + lane] = 0.0f;
+  int bad = 0;
+  const float4 *pv = reinterpret_cast<const float4 *>(piv);
+  const float4 *mv = reinterpret_cast<const float4 *>(mul);
+  *reinterpret_cast<float4 *>(piv + 4 * lane) = make_float4(c[0], c[1], c[2], c[3]);
+  __syncwarp();
+  LeafPivots f;
+  {
+    const float c4[4] = {c[0], c[1], c[2], c[3]};
+    f = leaf_pivots(pv[0], pv[1], pv[2], pv[3], c4);
+  }
+#pragma unroll 1
+  for (int k0 = 0; k0 < 32; k0 += 4) {
+    bad |= f.bad;  // (not the pivots formed past the last row)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int k = k0 + m;
+      if (lane < k) f.v[m] = 0.0f;  // left of the diagonal
+      if (lane == k && ((f.bad >> m) & 1)) f.v[m] = 1.0f;
+      S[(P + k) * LLD + P + lane] = f.v[m];
+      if (lane > k) shifted[k * LRD + lane - k - 1] = f.v[m];
+      if (lane == k) rd[P + k] = f.inv[m];
+    }
+    __syncwarp();  // the last step's readers of mul are done
+    *reinterpret_cast<float4 *>(mul + 4 * lane) = make_float4(f.v[0], f.v[1], f.v[2], f.v[3]);
+    __syncwarp();
+    // rows k0 + 4 .. k0 + 7 first: their pivot chain overlaps the other rows
+    float c4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 m = mv[k0 + 4 + i];
+      c4[i] = fmaf(-m.w, f.v[3], fmaf(-m.z, f.v[2], fmaf(-m.y, f.v[1],
+                                                         fmaf(-m.x, f.v[0], c[4 + i]))));
+    }
+    *reinterpret_cast<float4 *>(piv + 4 * lane) = make_float4(c4[0], c4[1], c4[2], c4[3]);
+    __syncwarp();
+    const int k1 = (k0 + 4) & 31;
+    const LeafPivots next = leaf_pivots(pv[k1], pv[k1 + 1], pv[k1 + 2], pv[k1 + 3], c4);
+#pragma unroll
+    for (int i = 8; i < 32; ++i) {
+      const float4 m = mv[k0 + i];  // rows past the block: zeros, never used
+      c[i - 4] = fmaf(-m.w, f.v[3], fmaf(-m.z, f.v[2], fmaf(-m.y, f.v[1],
+                                                            fmaf(-m.x, f.v[0], c[i]))));
+    }
+    f = next;
+  }
+  return bad != 0;
+}
+
+// (d): X_pp = U_pp^-1 by back substitution, lane l solving U x = e_l; x[q] holds row
+// i + 1 + q at row i (rows past the block are 0).  Four rows per body, so the rows
+// shift four registers at a time.  Returns max |X| over the valid columns.
+__device__ __forceinline__ float leaf_invert32(float *X, int P, const float *shifted,
+                                               const float *rd, int mp) {
+  const int lane = threadIdx.x & 31;
+  float am = 0.0f;
+  float x[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) x[i] = 0.0f;
+#pragma unroll 1
+  for (int s = 0; s < 32; s += 4) {
+    float n[4];  // the body's rows, newest first
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int i = 31 - s - m;
+      const float4 *row = reinterpret_cast<const float4 *>(shifted + i * LRD);
+      float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int q4 = 0; q4 < 8; ++q4) {
+        const float4 u4 = row[q4];
+        const float u[4] = {u4.x, u4.y, u4.z, u4.w};
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int q = 4 * q4 + t;  // row i + 1 + q: q < m from this body
+          if (q < m) a[t] = fmaf(u[t], n[m - 1 - q], a[t]);
+          else if (q - m < 32) a[t] = fmaf(u[t], x[q - m], a[t]);
+        }
+      }
+      const float ri = rd[P + i];
+      const float xi = (i == lane) ? ri : (i < lane ? -((a[0] + a[1]) + (a[2] + a[3])) * ri : 0.0f);
+      X[(P + i) * LLD + P + lane] = xi;
+      if (P + lane < mp) am = fmaxf(am, fabsf(xi));
+      n[m] = xi;
+    }
+#pragma unroll
+    for (int q = 31; q >= 4; --q) x[q] = x[q - 4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) x[q] = n[3 - q];
+  }
+  return am;
+}
+
+// Threads of two (b: 2) or four warps.
+__device__ __forceinline__ void leaf_sync_pair() { asm volatile("bar.sync 2, 64;" ::: "memory"); }
+__device__ __forceinline__ void leaf_sync_four() { asm volatile("bar.sync 3, 128;" ::: "memory"); }
+
+// 2 x 4 outputs (rows r2 .., columns c4 ..) of A B, K a multiple of 4: A row-major
+// (ld la), B row-major (ld lb).
+__device__ __forceinline__ void leaf_product(const float *A, int la, const float *B, int lb,
+                                             int K, int r2, int c4, float (&acc)[2][4]) {
+  const float *ar = A + r2 * la, *bc = B + c4;
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[r][q] = 0.0f;
+#pragma unroll 4
+  for (int k = 0; k < K; k += 4) {
+    const float4 a0 = *reinterpret_cast<const float4 *>(ar + k);
+    const float4 a1 = *reinterpret_cast<const float4 *>(ar + la + k);
+    const float x0[4] = {a0.x, a0.y, a0.z, a0.w}, x1[4] = {a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const float4 v = *reinterpret_cast<const float4 *>(bc + (k + m) * lb);
+      acc[0][0] = fmaf(x0[m], v.x, acc[0][0]);
+      acc[0][1] = fmaf(x0[m], v.y, acc[0][1]);
+      acc[0][2] = fmaf(x0[m], v.z, acc[0][2]);
+      acc[0][3] = fmaf(x0[m], v.w, acc[0][3]);
+      acc[1][0] = fmaf(x1[m], v.x, acc[1][0]);
+      acc[1][1] = fmaf(x1[m], v.y, acc[1][1]);
+      acc[1][2] = fmaf(x1[m], v.z, acc[1][2]);
+      acc[1][3] = fmaf(x1[m], v.w, acc[1][3]);
+    }
+  }
+}
+
+// S(i0 .., j0 ..) -= U(P .., i0 ..)^T U(P .., j0 ..), a 4 x 4 tile.  (Below the
+// diagonal of a diagonal block: entries nothing reads.)
+__device__ __forceinline__ void leaf_update_tile(float *S, int P, int i0, int j0) {
+  float acc[4][4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const float4 v = *reinterpret_cast<const float4 *>(S + (i0 + r) * LLD + j0);
+    acc[r][0] = v.x, acc[r][1] = v.y, acc[r][2] = v.z, acc[r][3] = v.w;
+  }
+#pragma unroll 4
+  for (int k = 0; k < 32; ++k) {
+    const float *row = S + (P + k) * LLD;
+    const float4 av = *reinterpret_cast<const float4 *>(row + i0);
+    const float4 bv = *reinterpret_cast<const float4 *>(row + j0);
+    const float a[4] = {av.x, av.y, av.z, av.w}, bq[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(-a[r], bq[q], acc[r][q]);
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    *reinterpret_cast<float4 *>(S + (i0 + r) * LLD + j0) =
+        make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+}
 
 __global__ void __launch_bounds__(LEAF_T, 1) chol_leaf_kernel(float *__restrict__ A, int64_t n,
                                                            int64_t r0, int mp,
@@ -476,232 +730,135 @@ __global__ void __launch_bounds__(LEAF_T, 1) chol_leaf_kernel(float *__restrict_
                                                            __half *__restrict__ xl,
                                                            float *scale_x, float *__restrict__ yinv,
                                                            int32_t *status) {
-  extern __shared__ float lsm[];
-  float *S = lsm;             // S[i * LLD + j] = U(i, j), i <= j; zero below
-  float *X = lsm + LB * LLD + LPAD;  // X[i * LLD + j] = U^-1(i, j), blocks I <= J only
-  float *rd = X + LB * LLD;          // rd[i] = 1 / U(i, i)
-  float *Tb = rd + LB;        // 3 x [32][33] temporaries of the inverse
+  extern __shared__ __align__(16) float lsm[];
+  float *S = lsm;                       // S[i * LLD + j]: A, then U(i, j), i <= j
+  float *X = S + LB * LLD;              // X[i * LLD + j] = U^-1(i, j), blocks I <= J only
+  float *shifted = X + LB * LLD;        // two panels' U_pp rows (factor / inversion overlap)
+  float *Tb = shifted + 2 * 32 * LRD;   // 3 x [32][LRD] temporaries of the inverse
+  float *rd = Tb + 3 * 32 * LRD;        // rd[i] = 1 / U(i, i)
+  float *piv = rd + LB;                 // 32 x float4: the four pivot rows' columns
+  float *mul = piv + 4 * 32;            // 64 x float4: four multipliers of each row
   __shared__ float red[LEAF_T / 32];
   __shared__ int not_spd;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) not_spd = 0;
-  if (tid < LPAD) S[LB * LLD + tid] = 0.0f;
+  for (int e = tid; e < 4 * 64; e += LEAF_T) mul[e] = 0.0f;
   pdl_wait();  // the block was written by the previous kernel of the stream
   pdl_trigger();
-  if (tid < LB) S[tid * LLD + LB] = 0.0f;  // each row's padding column
+  // lane = row i of block row warp & 3, columns 8 u + 4 (warp >> 2) + q
+  const int li = 32 * (warp & 3) + lane, lj = 4 * (warp >> 2);
   {
-    // all 64 of a thread's loads in flight at once
-    float v[LB * LB / LEAF_T];
+    float v[16][4];  // all of a thread's loads in flight at once
+    const float *col = A + (r0 + li) + (r0 + lj) * n;
 #pragma unroll
-    for (int u = 0; u < LB * LB / LEAF_T; ++u) {
-      const int e = u * LEAF_T + tid;
-      const int j = e / LB, i = e - j * LB;
-      v[u] = 0.0f;
-      if (i <= j) {
-        if (j < mp) v[u] = A[(r0 + i) + (r0 + j) * n];
-        else if (i == j) v[u] = 1.0f;
+    for (int u = 0; u < 16; ++u)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = lj + 8 * u + q;
+        v[u][q] = li == j ? 1.0f : 0.0f;
+        if (li <= j && j < mp) v[u][q] = col[(8 * u + q) * n];
       }
-    }
 #pragma unroll
-    for (int u = 0; u < LB * LB / LEAF_T; ++u) {
-      const int e = u * LEAF_T + tid;
-      const int j = e / LB, i = e - j * LB;
-      S[i * LLD + j] = v[u];
-    }
+    for (int u = 0; u < 16; ++u)
+      *reinterpret_cast<float4 *>(S + li * LLD + lj + 8 * u) =
+          make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
   }
-  __syncthreads();
+  leaf_sync_all();
+  float am = 0.0f;  // max |X| over the valid block (this thread's writes)
+  // off-diagonal block X_IJ by 128 threads (t)
+  auto x_block = [&](int I, int J, int t) {
+    const int r2 = 2 * (t >> 3), c4 = 4 * (t & 7);
+    float acc[2][4];
+    float *T = Tb + I * 32 * LRD;
+    leaf_product(S + 32 * I * LLD + 32 * (I + 1), LLD, X + 32 * (I + 1) * LLD + 32 * J, LLD,
+                 32 * (J - I), r2, c4, acc);
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      *reinterpret_cast<float4 *>(T + (r2 + r) * LRD + c4) =
+          make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+    leaf_sync_four();
+    leaf_product(X + 32 * I * LLD + 32 * I, LLD, T, LRD, 32, r2, c4, acc);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      *reinterpret_cast<float4 *>(X + (32 * I + r2 + r) * LLD + 32 * J + c4) =
+          make_float4(-acc[r][0], -acc[r][1], -acc[r][2], -acc[r][3]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (32 * J + c4 + q < mp) am = fmaxf(am, fabsf(acc[r][q]));
+    }
+    leaf_sync_four();
+  };
+  auto factor = [&](int p) {
+    if (leaf_factor32(S, 32 * p, shifted + (p & 1) * 32 * LRD, rd, piv, mul) && lane == 0)
+      not_spd = 1;
+  };
+  if (warp == 0) factor(0);
 #pragma unroll 1
   for (int p = 0; p < 4; ++p) {
     const int P = 32 * p;
-    if (warp == 0) {
-      // (a) at step k, c[i] holds row k + i of column P + lane
-      float c[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) c[i] = S[(P + i) * LLD + P + lane];
-      bool bad = false;
-      float d = __shfl_sync(0xffffffffu, c[0], 0);
-#pragma unroll 1
-      for (int k = 0; k < 32; ++k) {
-        if (!(d > 0.0f)) {
-          bad = true;
-          d = 1.0f;
-        }
-        const float inv = rsqrtf(d);
-        const float u = (lane == k) ? d * inv : (lane > k ? c[0] * inv : 0.0f);  // U(k, lane)
-        S[(P + k) * LLD + P + lane] = u;
-        if (lane == 0) rd[P + k] = inv;
-        // the next pivot's row first and its diagonal broadcast at once: the
-        // dependency from one pivot to the next is then these two steps, and
-        // the other 30 row updates issue while the broadcast is in flight
-        c[0] = fmaf(-__shfl_sync(0xffffffffu, u, (k + 1) & 31), u, c[1]);
-        const float dn = __shfl_sync(0xffffffffu, c[0], (k + 1) & 31);
-#pragma unroll
-        for (int i = 2; i < 32; ++i)
-          c[i - 1] = fmaf(-__shfl_sync(0xffffffffu, u, (k + i) & 31), u, c[i]);
-        c[31] = 0.0f;
-        d = dn;
-      }
-      if (bad && lane == 0) not_spd = 1;
+    leaf_sync_all();  // (a) of this panel and (c) of the last one are done
+    if (warp == 7) {
+      am = fmaxf(am, leaf_invert32(X, P, shifted + (p & 1) * 32 * LRD, rd, mp));
+      continue;
     }
-    __syncthreads();
     const int ncols = LB - P - 32;
-    if (ncols > 0) {
-      // (b) thread pair (2 jj, 2 jj + 1): column j, rows P + g + 2 r
-      if (tid < 2 * ncols) {
-        const int g = tid & 1, j = P + 32 + (tid >> 1);
-        float y[16];
+    if (ncols == 0) break;
+    // (b) one thread per column right of the block
+    if (tid < ncols) {
+      float *col = S + P * LLD + P + 32 + tid;
+      float y[32];
 #pragma unroll
-        for (int r = 0; r < 16; ++r) y[r] = S[(P + g + 2 * r) * LLD + j];
+      for (int r = 0; r < 32; ++r) y[r] = col[r * LLD];
 #pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          const float mine = (g == (k & 1)) ? y[k >> 1] * rd[P + k] : 0.0f;
-          const float yk = __shfl_sync(0xffffffffu, mine, (lane & ~1) | (k & 1));
-          if (g == (k & 1)) y[k >> 1] = yk;
-          const float *urow = S + (P + k) * LLD + P + g;  // U(k, P + g + 2 r) = urow[2 r]
-#pragma unroll
-          for (int r = 0; r < 16; ++r)
-            if (2 * r + 1 > k && 2 * r + g > k) y[r] = fmaf(-urow[2 * r], yk, y[r]);
-        }
-#pragma unroll
-        for (int r = 0; r < 16; ++r) S[(P + g + 2 * r) * LLD + j] = y[r];
-      }
-      __syncthreads();
-      // (c) trailing update of the upper triangle [P+32, 128)^2 in 4 x 4 tiles
-      const int T = ncols / 4, ntl = T * (T + 1) / 2;
-      const int base = P + 32;
-#pragma unroll 1
-      for (int t = tid; t < ntl; t += LEAF_T) {
-        int tj = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
-        while (tj * (tj + 1) / 2 > t) --tj;
-        while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
-        const int ti = t - tj * (tj + 1) / 2;
-        const int i0 = base + 4 * ti, j0 = base + 4 * tj;
-        float acc[4][4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[r][q] = S[(i0 + r) * LLD + j0 + q];
-#pragma unroll 4
-        for (int k = 0; k < 32; ++k) {
-          const float *row = S + (P + k) * LLD;
-          float a[4], bq[4];
-#pragma unroll
-          for (int r = 0; r < 4; ++r) a[r] = row[i0 + r];
-#pragma unroll
-          for (int q = 0; q < 4; ++q) bq[q] = row[j0 + q];
-#pragma unroll
-          for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(-a[r], bq[q], acc[r][q]);
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if (i0 + r <= j0 + q) S[(i0 + r) * LLD + j0 + q] = acc[r][q];
-      }
-      __syncthreads();
-    }
-  }
-  // diagonal blocks of X: warp p inverts U_pp; lane l solves U x = e_l from the
-  // bottom row up, x[q] holding row i + 1 + q at step s (i = 31 - s); rows past
-  // the block hold 0, so their products with the entries read past the block's
-  // last column (finite: later S entries, the zeroed padding column of each row
-  // or the zero pad after S) vanish
-  float am = 0.0f;  // max |X| over the valid block (this thread's writes)
-  if (warp < 4) {
-    const int P = 32 * warp;
-    float x[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) x[i] = 0.0f;
-#pragma unroll 1
-    for (int s2 = 0; s2 < 32; ++s2) {
-      const int i = 31 - s2;
-      const float *urow = S + (P + i) * LLD + P + i + 1;  // U(i, i + 1 + q) = urow[q]
-      float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-#pragma unroll
-      for (int q = 0; q < 32; q += 4) {
-        a0 = fmaf(urow[q], x[q], a0);
-        a1 = fmaf(urow[q + 1], x[q + 1], a1);
-        a2 = fmaf(urow[q + 2], x[q + 2], a2);
-        a3 = fmaf(urow[q + 3], x[q + 3], a3);
-      }
-      const float ri = rd[P + i];
-      const float xi = (i == lane) ? ri : (i < lane ? -((a0 + a1) + (a2 + a3)) * ri : 0.0f);
-      X[(P + i) * LLD + P + lane] = xi;
-      if (P + lane < mp) am = fmaxf(am, fabsf(xi));
-#pragma unroll
-      for (int q = 31; q > 0; --q) x[q] = x[q - 1];
-      x[0] = xi;
-    }
-  }
-  __syncthreads();
-  // off-diagonal blocks of X: X_IJ = -X_II sum_{K=I+1..J} U_IK X_KJ, by distance d
-  // (I = blk, J = blk + d), each thread a 4 x 4 tile of one block (64 per block)
-  // in registers.  X below the block diagonal is never read.
-#pragma unroll 1
-  for (int d = 1; d < 4; ++d) {
-    const int ntile = (4 - d) * 64;
-    const int blk = tid >> 6, r0t = 4 * ((tid >> 3) & 7), c0t = 4 * (tid & 7);
-    const bool act = tid < ntile;
-    float acc[4][4];
-    if (act) {
-      // phase 1: Tb[blk] = sum_K U_IK X_KJ over the 32 d columns right of block I
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[r][q] = 0.0f;
-      const float *ur = S + (32 * blk + r0t) * LLD + 32 * (blk + 1);
-      const float *xc = X + 32 * (blk + 1) * LLD + 32 * (blk + d) + c0t;
-#pragma unroll 4
-      for (int k = 0; k < 32 * d; ++k) {
-        float a[4], bq[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = ur[r * LLD + k];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) bq[q] = xc[k * LLD + q];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(a[r], bq[q], acc[r][q]);
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) Tb[blk * 32 * 33 + (r0t + r) * 33 + c0t + q] = acc[r][q];
-    }
-    __syncthreads();
-    if (act) {
-      // phase 2: X_IJ = -X_II Tb[blk]
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[r][q] = 0.0f;
-      const float *xr = X + (32 * blk + r0t) * LLD + 32 * blk;
-      const float *tc = Tb + blk * 32 * 33 + c0t;
-#pragma unroll 4
       for (int k = 0; k < 32; ++k) {
-        float a[4], bq[4];
+        y[k] *= rd[P + k];
+        const float *urow = S + (P + k) * LLD + P;  // U(k, r) = urow[r]
 #pragma unroll
-        for (int r = 0; r < 4; ++r) a[r] = xr[r * LLD + k];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) bq[q] = tc[k * 33 + q];
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[r][q] = fmaf(a[r], bq[q], acc[r][q]);
-      }
-      const int row0 = 32 * blk + r0t, col0 = 32 * (blk + d) + c0t;
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          X[(row0 + r) * LLD + col0 + q] = -acc[r][q];
-          if (col0 + q < mp) am = fmaxf(am, fabsf(acc[r][q]));
+        for (int r4 = 4 * (k / 4); r4 < 32; r4 += 4) {
+          const float4 u = *reinterpret_cast<const float4 *>(urow + r4);
+          if (r4 > k) y[r4] = fmaf(-u.x, y[k], y[r4]);
+          if (r4 + 1 > k) y[r4 + 1] = fmaf(-u.y, y[k], y[r4 + 1]);
+          if (r4 + 2 > k) y[r4 + 2] = fmaf(-u.z, y[k], y[r4 + 2]);
+          if (r4 + 3 > k) y[r4 + 3] = fmaf(-u.w, y[k], y[r4 + 3]);
         }
+      }
+#pragma unroll
+      for (int r = 0; r < 32; ++r) col[r * LLD] = y[r];
     }
-    __syncthreads();
+    leaf_sync_main();
+    // (c) the next diagonal block by warps 0 and 1, then warp 0 factors it
+    const int base = P + 32;
+    if (warp < 2) {
+      leaf_update_tile(S, P, base + 4 * (tid >> 3), base + 4 * (tid & 7));
+      leaf_sync_pair();
+    }
+    if (warp == 0) {
+      factor(p + 1);
+    } else {
+      // the other blocks (i <= j, not the first): 64 tiles each, warps 1 .. 6
+      const int below = 3 - p, tiles = 64 * (below * (below + 1) / 2 - 1);
+#pragma unroll 1
+      for (int t = tid - 32; t < tiles; t += 192) {
+        int blk = 1 + (t >> 6), bi = 0;
+        while (blk >= below - bi) blk -= below - bi++;
+        leaf_update_tile(S, P, base + 32 * bi + 4 * ((t >> 3) & 7),
+                         base + 32 * (bi + blk) + 4 * (t & 7));
+      }
+      // behind the last factor: X_01 (X_00 and X_11 are there)
+      if (p == 2 && warp >= 3) x_block(0, 1, tid - 96);
+    }
   }
+  // behind the last inversion: X_12 and X_02; then the last block column
+  if (warp < 4) {
+    x_block(1, 2, tid);
+    x_block(0, 2, tid);
+  }
+  leaf_sync_all();  // X_33 too
+  if (warp < 4) {
+#pragma unroll 1
+    for (int I = 2; I >= 0; --I) x_block(I, 3, tid);
+  }
+  leaf_sync_all();
   // max |X| over the valid block -> split scale
   for (int o = 16; o > 0; o >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, o));
   if (lane == 0) red[warp] = am;
@@ -714,26 +871,51 @@ __global__ void __launch_bounds__(LEAF_T, 1) chol_leaf_kernel(float *__restrict_
     *scale_x = sx;
     if (not_spd && status) atomicOr(status, VMCK_DEV_NOT_SPD);
   }
-  // outputs
-  for (int j = warp; j < mp; j += LEAF_T / 32)
-    for (int i = lane; i <= j; i += 32) A[(r0 + i) + (r0 + j) * n] = S[i * LLD + j];
-  for (int e = 2 * tid; e < LB * LB; e += 2 * LEAF_T) {
-    const int m = e / LB, k = e - m * LB;  // row m of the split operand = column m of X
-    __half h0 = __float2half_rn(0.0f), l0 = h0, h1 = h0, l1 = h0;
-    if (m < mp && k <= m) split_f16(X[k * LLD + m], sx, h0, l0);
-    if (m < mp && k + 1 <= m) split_f16(X[(k + 1) * LLD + m], sx, h1, l1);
-    reinterpret_cast<__half2 *>(xh)[e >> 1] = __halves2half2(h0, h1);
-    reinterpret_cast<__half2 *>(xl)[e >> 1] = __halves2half2(l0, l1);
+  // outputs.  X split: lane = two rows, four columns at a time; the blocks of the
+  // operand that are zero for every leaf were cleared once by the caller
+  for (int t = warp; t < 64; t += LEAF_T / 32) {
+    const int i = 64 * (t & 1) + 2 * lane, j0 = 4 * (t >> 1);
+    if (64 * (t & 1) > j0 + 3) continue;
+    const float4 x0 = *reinterpret_cast<const float4 *>(X + i * LLD + j0);
+    const float4 x1 = *reinterpret_cast<const float4 *>(X + (i + 1) * LLD + j0);
+    const float a[4] = {x0.x, x0.y, x0.z, x0.w}, c[4] = {x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = j0 + q;  // row j of the split operand = column j of X
+      __half h0 = __float2half_rn(0.0f), l0 = h0, h1 = h0, l1 = h0;
+      if (j < mp && i <= j) split_f16(a[q], sx, h0, l0);
+      if (j < mp && i + 1 <= j) split_f16(c[q], sx, h1, l1);
+      *reinterpret_cast<__half2 *>(xh + j * LB + i) = __halves2half2(h0, h1);
+      *reinterpret_cast<__half2 *>(xl + j * LB + i) = __halves2half2(l0, l1);
+    }
   }
-  for (int e = tid; e < LB * LB; e += LEAF_T) {
-    const int c = e / LB, r = e - c * LB;  // Y(r, c) = X(c, r)
-    yinv[e] = (r < mp && c <= r) ? X[c * LLD + r] : 0.0f;
+  {
+    float *col = A + (r0 + li) + (r0 + lj) * n;
+#pragma unroll 4
+    for (int u = 0; u < 16; ++u) {
+      if (32 * (warp & 3) > lj + 8 * u + 3) continue;  // below the diagonal
+      const float4 v = *reinterpret_cast<const float4 *>(S + li * LLD + lj + 8 * u);
+      const float us[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int j = lj + 8 * u + q;
+        if (li <= j && j < mp) col[(8 * u + q) * n] = us[q];
+      }
+    }
+  }
+  for (int c = warp; c < LB; c += LEAF_T / 32) {
+    const int r = 4 * lane;  // Y(r, c) = X(c, r); above the diagonal cleared by the caller
+    if (r + 3 < c) continue;
+    const float4 v = *reinterpret_cast<const float4 *>(X + c * LLD + r);
+    *reinterpret_cast<float4 *>(yinv + c * LB + r) =
+        make_float4(r < mp && c <= r ? v.x : 0.0f, r + 1 < mp && c <= r + 1 ? v.y : 0.0f,
+                    r + 2 < mp && c <= r + 2 ? v.z : 0.0f, r + 3 < mp && c <= r + 3 ? v.w : 0.0f);
   }
 }
 
 // ------------------------------------------------------------ host side
 static int make_f16_map(CUtensorMap *map, const __half *base, int64_t kdim, int64_t rows,
-                        int64_t ld) {
+                        int64_t ld, int box_rows) {
   auto fn = encode_fn();
   if (!fn) {
     set_last_error("cuTensorMapEncodeTiled is unavailable");
@@ -741,7 +923,7 @@ static int make_f16_map(CUtensorMap *map, const __half *base, int64_t kdim, int6
   }
   cuuint64_t dims[2] = {(cuuint64_t)kdim, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
-  cuuint32_t box[2] = {(cuuint32_t)G_BK, (cuuint32_t)G_BM};
+  cuuint32_t box[2] = {(cuuint32_t)G_BK, (cuuint32_t)box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(base), dims,
                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -761,7 +943,42 @@ static int num_sms_dev() {
   return sms;
 }
 
-static size_t gemm_smem_bytes() { return 1024 + G_STAGES * G_STAGE_BYTES + 8 * 16 + 64; }
+template <int BN>
+static int launch_gemm(cudaStream_t st, const SplitOperand &a, const SplitOperand &b,
+                       GemmParams g, int sms) {
+  CUtensorMap mAh, mAl, mBh, mBl;
+  int rc;
+  constexpr int box = GemmTile<BN>::BOX;
+  if ((rc = make_f16_map(&mAh, a.hi, a.kdim, a.rows, a.ld, G_BM))) return rc;
+  if ((rc = make_f16_map(&mAl, a.lo, a.kdim, a.rows, a.ld, G_BM))) return rc;
+  if ((rc = make_f16_map(&mBh, b.hi, b.kdim, b.rows, b.ld, box))) return rc;
+  if ((rc = make_f16_map(&mBl, b.lo, b.kdim, b.rows, b.ld, box))) return rc;
+  g.mt = (g.M + G_BM - 1) / G_BM;
+  g.nt = (g.N + BN - 1) / BN;
+  if (g.tri && g.mt > 1) {
+    const int64_t h = g.mt / 2;
+    g.base_tiles = g.nt <= h ? (int64_t)g.nt * (g.nt + 1) : h * (h + 1) + (int64_t)(g.nt - h) * g.mt;
+  } else {
+    g.base_tiles = (int64_t)g.mt * g.nt;
+  }
+  g.tiles = g.base_tiles * g.kz;
+  const size_t smem = 1024 + G_STAGES * GemmTile<BN>::STAGE_BYTES + 8 * 16 + 64;
+  VMCK_CUDA(cudaFuncSetAttribute(tc_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem));
+  const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, sms);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(G_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  VMCK_CUDA(cudaLaunchKernelEx(&cfg, tc_gemm_kernel<BN>, mAh, mAl, mBh, mBl, g));
+  return check_launch("tc_gemm");
+}
 
 int tc_gemm(cudaStream_t st, const SplitOperand &a, int a_row0, const SplitOperand &b, int b_row0,
             int k_off, int M, int N, int K, float *C, int64_t ldc, float alpha, float beta,
@@ -774,12 +991,6 @@ int tc_gemm(cudaStream_t st, const SplitOperand &a, int a_row0, const SplitOpera
     set_last_error("tc_gemm: split K needs kchunk %% %d == 0, no tri / split output / beta", G_BK);
     return VMCK_ERR_ARG;
   }
-  CUtensorMap mAh, mAl, mBh, mBl;
-  int rc;
-  if ((rc = make_f16_map(&mAh, a.hi, a.kdim, a.rows, a.ld))) return rc;
-  if ((rc = make_f16_map(&mAl, a.lo, a.kdim, a.rows, a.ld))) return rc;
-  if ((rc = make_f16_map(&mBh, b.hi, b.kdim, b.rows, b.ld))) return rc;
-  if ((rc = make_f16_map(&mBl, b.lo, b.kdim, b.rows, b.ld))) return rc;
   GemmParams g{};
   g.M = M;
   g.N = N;
@@ -803,35 +1014,15 @@ int tc_gemm(cudaStream_t st, const SplitOperand &a, int a_row0, const SplitOpera
   g.so = so;
   g.status = status;
   g.wait_ns = wait_limit_ns();
-  g.mt = (M + G_BM - 1) / G_BM;
-  g.nt = (N + G_BN - 1) / G_BN;
-  if (tri) {
-    const int64_t h = g.mt / 2;
-    g.base_tiles = g.nt <= h ? (int64_t)g.nt * (g.nt + 1) : h * (h + 1) + (int64_t)(g.nt - h) * g.mt;
-  } else {
-    g.base_tiles = (int64_t)g.mt * g.nt;
-  }
   g.kchunk = kchunk;
   g.kz = (K + kchunk - 1) / kchunk;
   g.zstride = zstride;
-  g.tiles = g.base_tiles * g.kz;
-  const size_t smem = gemm_smem_bytes();
-  VMCK_CUDA(cudaFuncSetAttribute(tc_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
   const int sms = max_ctas > 0 ? max_ctas : num_sms_dev();
-  const unsigned grid = (unsigned)std::min<int64_t>(g.tiles, sms);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(G_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  VMCK_CUDA(cudaLaunchKernelEx(&cfg, tc_gemm_kernel, mAh, mAl, mBh, mBl, g));
-  return check_launch("tc_gemm");
+  if (M <= G_BM && g.kz == 1) {
+    if (N <= 64 * sms) return launch_gemm<64>(st, a, b, g, sms);
+    if (N <= 128 * sms) return launch_gemm<128>(st, a, b, g, sms);
+  }
+  return launch_gemm<256>(st, a, b, g, sms);
 }
 
 int chol_block_rows(int64_t n) {
@@ -935,6 +1126,10 @@ int chol_tc_factor(cudaStream_t st, float *A, int64_t n, void *ws, int32_t *stat
   const int side_grid = two ? side_ctas(num_sms_dev(), n) : 0;
   VMCK_CUDA(cudaFuncSetAttribute(chol_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)CHOL_LEAF_SMEM));
+  // the leaf writes X and Y on and above, or below, their diagonals
+  VMCK_CUDA(cudaMemsetAsync(yinv, 0, (size_t)((n + LB - 1) / LB) * LB * LB * 4, chain));
+  VMCK_CUDA(cudaMemsetAsync(xs_hi, 0, (size_t)LB * LB * 2, chain));
+  VMCK_CUDA(cudaMemsetAsync(xs_lo, 0, (size_t)LB * LB * 2, chain));
   chol_bounds_kernel<<<1, 256, 0, chain>>>(A, n, scales, status);
   if ((rc = check_launch("chol_tc bounds"))) return rc;
   {
