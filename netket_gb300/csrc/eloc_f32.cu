@@ -15,8 +15,8 @@
 // through L1.  Each warp lists the connected elements of its share of the terms
 // by ballots, with nothing shared between warps before the sample's sum.
 //
-// What bounds it: FP32 issue (18 instructions per 32 hidden units of an element).
-// 10 x 10 J1-J2, M = 400, n = 16,384 (about 200 elements a sample): @LOCAL@.
+// What bounds it: FP32 issue (27 instructions per 32 hidden units of an element).
+// 10 x 10 J1-J2, M = 400, n = 16,384 (about 200 elements a sample): 2.10 -> 1.17 ms.
 #include <algorithm>
 
 #include "eloc_f32.cuh"

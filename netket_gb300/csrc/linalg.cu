@@ -18,6 +18,7 @@
 
 #include "chol_tc.cuh"
 #include "common.cuh"
+#include "tc_common.cuh"
 
 struct vmck_ctx {
   int device = 0;
@@ -697,16 +698,25 @@ __global__ void __launch_bounds__(LEAF_THREADS) trsm_leaf_kernel(const float *__
 
 // ------------------------------------------------------------ blocked triangular solves
 // U^T y = r and U x = y for the FP32 upper factor U (column-major, ld n) in
-// 128-row blocks, for the refinement loop.  trsv_inv_kernel stores
-// Y_K = U_KK^-T (lower, column-major 128 x 128, zero-padded) for every diagonal
-// block, so a block's own solve is a 128 x 128 product.  The two solve kernels
-// are persistent: CTAs take block tickets in order from an atomic counter, so
-// every block a CTA waits for has been claimed by a CTA that is already running
-// and that never waits for a later block; a finished block is published with a
-// release store of the call's epoch into its flag.  Waits are bounded (the
-// library's wait limit, 2 s of wall time by default); a wait that runs out raises
-// VMCK_DEV_TIMEOUT and sets the abort word, which makes every other wait give up
-// at once.  A CTA holds nothing when it gives up (no copies or MMAs in flight).
+// 128-row blocks, for the refinement loop.  Y_K = U_KK^-T (lower, column-major
+// 128 x 128, zero-padded) is kept for every diagonal block, so a block's own solve
+// is a 128 x 128 product.  The two solve kernels are persistent: CTAs take block
+// tickets in order from an atomic counter, so every block a CTA waits for has been
+// claimed by a CTA that is already running and that never waits for a later block.
+//
+// The chain of blocks bounds them (128 blocks at n = 16,384, 0.54 GB of U): a block
+// is published as 64-bit words {epoch, value}, one store per entry, and the CTAs
+// that wait poll the words themselves, so a hand-over is one store and one load
+// instead of data, fence, flag, flag read and data read.  A seventeenth warp polls
+// ahead into a ring of shared-memory slots while the other sixteen multiply, with
+// the next block's part of U already on its way to registers.  n = 4,096 / 16,384:
+// Forward 405 -> 205 us and backward 425 -> 190 us at n = 16,384; 91 -> 48 and 79 -> 42 us
+// at n = 4,096.
+//
+// Waits are bounded (the library's wait limit, 2 s of wall time by default); a wait
+// that runs out raises VMCK_DEV_TIMEOUT and sets the abort word, which makes every
+// other wait give up at once.  A CTA holds nothing when it gives up (no copies or
+// MMAs in flight).
 constexpr int TB = 128;
 
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
@@ -714,28 +724,10 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_u32(unsigned *p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ unsigned long long wall_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
-}
-
-// Every lane of the warp spins; returns false if the solve was aborted.
-__device__ __forceinline__ bool trsv_wait(const unsigned *flag, unsigned epoch, unsigned *abort_w,
-                          int32_t *status, unsigned long long limit) {
-  const unsigned long long t0 = wall_ns();
-  for (unsigned it = 0;; ++it) {
-    if (ld_acquire_u32(flag) == epoch) return true;
-    if (ld_acquire_u32(abort_w) == epoch) return false;
-    if (it >= 4 && wall_ns() - t0 > limit) {
-      if (status) atomicOr(status, VMCK_DEV_TIMEOUT);
-      atomicExch(abort_w, epoch);
-      return false;
-    }
-  }
 }
 
 __global__ void __launch_bounds__(LEAF_THREADS) trsv_inv_kernel(const float *__restrict__ U,
@@ -766,174 +758,307 @@ __global__ void __launch_bounds__(LEAF_THREADS) trsv_inv_kernel(const float *__r
 }
 
 struct TrsvSync {
-  unsigned *flags;   // nb
-  unsigned *ticket;  // 1
-  unsigned *abort_w; // 1
+  unsigned *ticket;        // this kernel's blocks
+  unsigned *other_ticket;  // the other direction's, cleared for its next launch
+  unsigned *abort_w;
   unsigned long long wait_ns;  // limit of each wait
 };
 
-// y = U^-T r.  Block K: z = r_K - sum_{J<K} U_JK^T y_J (warp w: columns 8w..8w+7 of
-// block K, each a 128-long contiguous column segment per J), then y_K = Y_K z.
-__global__ void __launch_bounds__(LEAF_THREADS) trsv_fwd_kernel(const float *__restrict__ U,
-                                                                int64_t n,
-                                                                const float *__restrict__ Yinv,
-                                                                const float *__restrict__ r,
-                                                                float *y, TrsvSync sy,
-                                                                unsigned epoch, int32_t *status,
-                                                                const int *done) {
+constexpr int TRSV_WARPS = 16, TRSV_THREADS = 32 * (TRSV_WARPS + 1), TRSV_SLOTS = 4;
+constexpr size_t TRSV_SMEM = (size_t)TB * TB * 4;  // Y_K of the forward solve
+
+// {epoch, value} words: written and read whole, so a word with the call's epoch
+// carries its value.
+__device__ __forceinline__ void trsv_put(unsigned long long *p, float v, unsigned epoch) {
+  const unsigned long long w = (unsigned long long)epoch << 32 | __float_as_uint(v);
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+__device__ __forceinline__ float trsv_value(unsigned long long w) {
+  return __uint_as_float((unsigned)w);
+}
+
+// The warp's 128 words of a block, lane l words 4 l .. 4 l + 3 (src: the lane's
+// first); false (on every lane) when the solve was aborted or the wait ran out.
+__device__ __forceinline__ bool trsv_poll(const unsigned long long *src, unsigned epoch,
+                                          const TrsvSync &sy, int32_t *status, float4 &out) {
+  const unsigned long long t0 = wall_ns();
+  for (unsigned it = 0;; ++it) {
+    unsigned long long w[4];
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                 : "=l"(w[0]), "=l"(w[1]) : "l"(src) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                 : "=l"(w[2]), "=l"(w[3]) : "l"(src + 2) : "memory");
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ok &= (unsigned)(w[q] >> 32) == epoch;
+    if (__all_sync(0xffffffffu, ok)) {
+      out = make_float4(trsv_value(w[0]), trsv_value(w[1]), trsv_value(w[2]), trsv_value(w[3]));
+      return true;
+    }
+    const bool late = it >= 4 && wall_ns() - t0 > sy.wait_ns;
+    if (__any_sync(0xffffffffu, late)) {
+      if ((threadIdx.x & 31) == 0) {
+        if (status) atomicOr(status, VMCK_DEV_TIMEOUT);
+        atomicExch(sy.abort_w, epoch);
+      }
+      return false;
+    }
+    if (__any_sync(0xffffffffu, ld_acquire_u32(sy.abort_w) == epoch)) return false;
+  }
+}
+
+// What a solve kernel's CTA shares: the ring of polled blocks and its barriers.
+struct TrsvRing {
+  float4 slot[TRSV_SLOTS][32];
+  uint64_t full[TRSV_SLOTS], empty[TRSV_SLOTS];
+  int block, abort;
+};
+
+__device__ __forceinline__ void trsv_ring_init(TrsvRing &r, const TrsvSync &sy) {
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < TRSV_SLOTS; ++s) {
+      mbar_init(&r.full[s], 32);
+      mbar_init(&r.empty[s], TRSV_WARPS);
+    }
+    r.abort = 0;
+    if (blockIdx.x == 0) *sy.other_ticket = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+}
+
+// The polling warp's part: `count` blocks, the first at p, then p + step, ...; `it`
+// counts the blocks of the launch.
+__device__ __forceinline__ void trsv_feed(TrsvRing &r, const unsigned long long *p, int64_t step,
+                                          int count, unsigned &it, unsigned epoch,
+                                          const TrsvSync &sy, int32_t *status) {
+  const int lane = threadIdx.x & 31;
+  for (int q = 0; q < count; ++q, ++it, p += step) {
+    const unsigned s = it % TRSV_SLOTS;
+    bool ok = it < TRSV_SLOTS ||
+              mbar_wait(&r.empty[s], (it / TRSV_SLOTS - 1) & 1, sy.wait_ns + TC_DRAIN_NS);
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    ok = __all_sync(0xffffffffu, ok) && trsv_poll(p + 4 * lane, epoch, sy, status, v);
+    if (ok) r.slot[s][lane] = v;
+    else r.abort = 1;
+    mbar_arrive(&r.full[s]);
+    if (!ok) return;
+  }
+}
+
+// The other warps' wait for block `it`; false when the solve was aborted.
+__device__ __forceinline__ bool trsv_take(TrsvRing &r, unsigned it, const TrsvSync &sy,
+                                          int32_t *status) {
+  if (!mbar_wait(&r.full[it % TRSV_SLOTS], (it / TRSV_SLOTS) & 1,
+                 2 * (sy.wait_ns + TC_DRAIN_NS))) {
+    if (status) atomicOr(status, VMCK_DEV_TIMEOUT);
+    r.abort = 1;
+    return false;
+  }
+  return *reinterpret_cast<volatile int *>(&r.abort) == 0;
+}
+__device__ __forceinline__ void trsv_release(TrsvRing &r, unsigned it) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(&r.empty[it % TRSV_SLOTS]);
+}
+
+// Warp sums of eight values per lane, in warp_sum's order (l ^ 16, 8, 4, 2, 1): the
+// sum of value q = 4 (l >> 4) + 2 (l >> 3 & 1) + (l >> 2 & 1) on lane l, in nine
+// exchanges instead of forty.
+__device__ __forceinline__ float warp_sum8(const float (&v)[8], int &q) {
+  const int lane = threadIdx.x & 31;
+  const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+  float a[4], b[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    a[i] = (h16 ? v[4 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[4 + i], 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    b[i] = (h8 ? a[2 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, h8 ? a[i] : a[2 + i], 8);
+  float c = (h4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[1], 4);
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 1);
+  q = (h16 ? 4 : 0) + (h8 ? 2 : 0) + (h4 ? 1 : 0);
+  return c;
+}
+
+// y = U^-T fp32(r) (r has n_real entries, zeros up to n).  Block K: z = r_K -
+// sum_{J<K} U_JK^T y_J (warp w: columns 8w..8w+7 of block K, each a 128-long
+// contiguous column segment per J), then y_K = Y_K z.
+__global__ void __launch_bounds__(TRSV_THREADS, 1)
+    trsv_fwd_kernel(const float *__restrict__ U, int64_t n, const float *__restrict__ Yinv,
+                    const double *__restrict__ r, int64_t n_real, unsigned long long *yp,
+                    TrsvSync sy, unsigned epoch, int32_t *status, const int *done) {
   if (refine_done(done)) return;  // before any ticket: every CTA leaves
-  __shared__ float z[TB];
+  extern __shared__ __align__(16) float ysm[];  // Y_K, column-major
+  __shared__ TrsvRing ring;
+  __shared__ __align__(16) float z[TB];
   __shared__ float part[4][TB];
-  __shared__ int K_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nb = (int)((n + TB - 1) / TB);
+  trsv_ring_init(ring, sy);
+  unsigned it = 0;
   while (true) {
     __syncthreads();
-    if (tid == 0) K_s = (int)atomicAdd(sy.ticket, 1u);
+    if (tid == 0) ring.block = (int)atomicAdd(sy.ticket, 1u);
     __syncthreads();
-    const int K = K_s;
+    const int K = ring.block;
     if (K >= nb) break;
     const int64_t k0 = (int64_t)K * TB;
     const int mk = (int)((n - k0) < TB ? (n - k0) : TB);
-    // this thread's share of Y_K for the final product, loaded before any wait
-    const int yc = tid & (TB - 1), yh = tid >> 7;
-    float ys[32];
-    {
-      const float *Y = Yinv + (int64_t)K * TB * TB;
+    const int yc = tid & (TB - 1), yh = (tid >> 7) & 3;
+    if (warp == TRSV_WARPS) {
+      trsv_feed(ring, yp, TB, K, it, epoch, sy, status);
+    } else {
+      // Y_K for the final product and this lane's entry of r, loaded before any wait
+      const float4 *Y = reinterpret_cast<const float4 *>(Yinv + (int64_t)K * TB * TB);
 #pragma unroll
-      for (int i = 0; i < 32; ++i) ys[i] = __ldg(Y + (32 * yh + i) * TB + yc);
-    }
-    float acc[8] = {};
-    bool alive = true;
-    for (int J = 0; J < K && alive; ++J) {
-      float4 u[8];  // U_JK does not depend on y: load it before waiting for y_J
+      for (int i = 0; i < 8; ++i)
+        reinterpret_cast<float4 *>(ysm)[tid + 512 * i] = __ldg(Y + tid + 512 * i);
+      const int qc = 8 * warp + ((lane >> 4) << 2) + ((lane >> 2) & 2) + ((lane >> 2) & 1);
+      const float rc = k0 + qc < n_real ? (float)r[k0 + qc] : 0.0f;
+      float acc[8] = {};
+      float4 u[8];
+      auto load_u = [&](int J) {  // U_JK does not depend on y
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int c = 8 * warp + q;
-        u[q] = (c < mk) ? __ldg(reinterpret_cast<const float4 *>(U + (k0 + c) * n + (int64_t)J * TB) + lane)
-                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int q = 0; q < 8; ++q) {
+          const int c = 8 * warp + q;
+          u[q] = (c < mk) ? __ldg(reinterpret_cast<const float4 *>(U + (k0 + c) * n +
+                                                                   (int64_t)J * TB) + lane)
+                          : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+      };
+      if (K > 0) load_u(0);
+      for (int J = 0; J < K; ++J, ++it) {
+        if (!trsv_take(ring, it, sy, status)) break;
+        const float4 yj = ring.slot[it % TRSV_SLOTS][lane];
+        trsv_release(ring, it);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          acc[q] = __fmaf_rn(u[q].x, yj.x, __fmaf_rn(u[q].y, yj.y, __fmaf_rn(u[q].z, yj.z, __fmaf_rn(u[q].w, yj.w, acc[q]))));
+        if (J + 1 < K) load_u(J + 1);
       }
-      alive = trsv_wait(sy.flags + J, epoch, sy.abort_w, status, sy.wait_ns);
-      if (!alive) break;
-      const float4 yj = __ldcg(reinterpret_cast<const float4 *>(y + (int64_t)J * TB) + lane);
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        acc[q] = __fmaf_rn(u[q].x, yj.x, __fmaf_rn(u[q].y, yj.y, __fmaf_rn(u[q].z, yj.z, __fmaf_rn(u[q].w, yj.w, acc[q]))));
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float v = warp_sum(acc[q]);
-      const int c = 8 * warp + q;
-      if (lane == 0) z[c] = (c < mk) ? r[k0 + c] - v : 0.0f;
+      int q;
+      const float v = warp_sum8(acc, q);
+      if ((lane & 3) == 0) z[8 * warp + q] = (8 * warp + q < mk) ? rc - v : 0.0f;
     }
     __syncthreads();
-    {  // y_K[c] = sum_c' Y_K(c, c') z[c'], thread (h, c): c' in [32h, 32h + 32)
+    if (ring.abort) return;
+    if (warp < TRSV_WARPS) {  // y_K[c] = sum_c' Y_K(c, c') z[c'], thread (h, c): c' in [32h, 32h + 32)
       float sacc = 0.0f;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) sacc = __fmaf_rn(ys[i], z[32 * yh + i], sacc);
+      for (int i = 0; i < 32; i += 4) {
+        const float4 z4 = *reinterpret_cast<const float4 *>(z + 32 * yh + i);
+        const float *y = ysm + (32 * yh + i) * TB + yc;
+        sacc = __fmaf_rn(y[0], z4.x, sacc);
+        sacc = __fmaf_rn(y[TB], z4.y, sacc);
+        sacc = __fmaf_rn(y[2 * TB], z4.z, sacc);
+        sacc = __fmaf_rn(y[3 * TB], z4.w, sacc);
+      }
       part[yh][yc] = sacc;
     }
     __syncthreads();
-    if (tid < mk) {
-      __stcg(y + k0 + tid, (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]));
-      __threadfence();
-    }
-    __syncthreads();
-    if (tid == 0) st_release_u32(sy.flags + K, epoch);
+    if (tid < TB)
+      trsv_put(yp + k0 + tid,
+               tid < mk ? (part[0][tid] + part[1][tid]) + (part[2][tid] + part[3][tid]) : 0.0f,
+               epoch);
   }
 }
 
 // x = U^-1 y.  Block K (taken from the last): w = y_K - sum_{J>K} U_KJ x_J (warp w:
 // columns 8w..8w+7 of every later block J; lane: rows 4 lane..4 lane+3), then
-// x_K = Y_K^T w.
-__global__ void __launch_bounds__(LEAF_THREADS) trsv_bwd_kernel(const float *__restrict__ U,
-                                                                int64_t n,
-                                                                const float *__restrict__ Yinv,
-                                                                const float *__restrict__ yv,
-                                                                float *x, TrsvSync sy,
-                                                                unsigned epoch, int32_t *status,
-                                                                const int *done) {
+// x_K = Y_K^T w, stored in x (nullable) and added to x64 (nullable; n_real entries).
+__global__ void __launch_bounds__(TRSV_THREADS, 1)
+    trsv_bwd_kernel(const float *__restrict__ U, int64_t n, const float *__restrict__ Yinv,
+                    const unsigned long long *__restrict__ yp, unsigned long long *xp, float *x,
+                    double *x64, int64_t n_real, TrsvSync sy, unsigned epoch, int32_t *status,
+                    const int *done) {
   if (refine_done(done)) return;
+  __shared__ TrsvRing ring;
   __shared__ __align__(16) float wv[TB];
   __shared__ float part[16][TB];
-  __shared__ int K_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nb = (int)((n + TB - 1) / TB);
+  trsv_ring_init(ring, sy);
+  unsigned it = 0;
   while (true) {
     __syncthreads();
-    if (tid == 0) K_s = nb - 1 - (int)atomicAdd(sy.ticket, 1u);
+    if (tid == 0) ring.block = nb - 1 - (int)atomicAdd(sy.ticket, 1u);
     __syncthreads();
-    const int K = K_s;
+    const int K = ring.block;
     if (K < 0) break;
     const int64_t k0 = (int64_t)K * TB;
     const int mk = (int)((n - k0) < TB ? (n - k0) : TB);
-    const bool full = (4 * lane + 3) < mk;
-    // this warp's columns of Y_K for the final product, loaded before any wait
     float4 ycol[8];
-    {
+    float yk = 0.0f;
+    if (warp == TRSV_WARPS) {
+      trsv_feed(ring, xp + (int64_t)(nb - 1) * TB, -TB, nb - 1 - K, it, epoch, sy, status);
+    } else {
+      // this warp's columns of Y_K for the final product, loaded before any wait
       const float *Y = Yinv + (int64_t)K * TB * TB;
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         ycol[q] = __ldg(reinterpret_cast<const float4 *>(Y + (int64_t)(8 * warp + q) * TB) + lane);
-    }
-    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-    bool alive = true;
-    for (int J = nb - 1; J > K && alive; --J) {
-      const int64_t j0 = (int64_t)J * TB;
-      const int mj = (int)((n - j0) < TB ? (n - j0) : TB);
-      float4 u[8];  // U_KJ does not depend on x: load it before waiting for x_J
+      if (tid < mk) yk = trsv_value(yp[k0 + tid]);
+      float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+      float4 u[8];
+      auto load_u = [&](int J) {  // U_KJ does not depend on x; block K is full (J > K)
+        const int64_t j0 = (int64_t)J * TB;
+        const int mj = (int)((n - j0) < TB ? (n - j0) : TB);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int cj = 8 * warp + q;
-        const float *col = U + (j0 + cj) * n + k0;
-        if (cj >= mj) {
-          u[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        } else if (full) {
-          u[q] = __ldg(reinterpret_cast<const float4 *>(col) + lane);
-        } else {
-          const int rr = 4 * lane;
-          u[q] = make_float4(rr < mk ? col[rr] : 0.0f, rr + 1 < mk ? col[rr + 1] : 0.0f,
-                             rr + 2 < mk ? col[rr + 2] : 0.0f, 0.0f);
+        for (int q = 0; q < 8; ++q) {
+          const int cj = 8 * warp + q;
+          u[q] = cj < mj ? __ldg(reinterpret_cast<const float4 *>(U + (j0 + cj) * n + k0) + lane)
+                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
-      }
-      alive = trsv_wait(sy.flags + J, epoch, sy.abort_w, status, sy.wait_ns);
-      if (!alive) break;
+      };
+      if (K < nb - 1) load_u(nb - 1);
+      for (int J = nb - 1; J > K; --J, ++it) {
+        if (!trsv_take(ring, it, sy, status)) break;
+        const float4 *sl = ring.slot[it % TRSV_SLOTS];
+        const float4 x0 = sl[2 * warp], x1 = sl[2 * warp + 1];
+        trsv_release(ring, it);
+        // entries past the last block's end were published as zeros
+        const float xj[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float xj = (8 * warp + q < mj) ? __ldcg(x + j0 + 8 * warp + q) : 0.0f;
-        a0 = __fmaf_rn(u[q].x, xj, a0);
-        a1 = __fmaf_rn(u[q].y, xj, a1);
-        a2 = __fmaf_rn(u[q].z, xj, a2);
-        a3 = __fmaf_rn(u[q].w, xj, a3);
+        for (int q = 0; q < 8; ++q) {
+          a0 = __fmaf_rn(u[q].x, xj[q], a0);
+          a1 = __fmaf_rn(u[q].y, xj[q], a1);
+          a2 = __fmaf_rn(u[q].z, xj[q], a2);
+          a3 = __fmaf_rn(u[q].w, xj[q], a3);
+        }
+        if (J - 1 > K) load_u(J - 1);
       }
+      part[warp][4 * lane] = a0;
+      part[warp][4 * lane + 1] = a1;
+      part[warp][4 * lane + 2] = a2;
+      part[warp][4 * lane + 3] = a3;
     }
-    part[warp][4 * lane] = a0;
-    part[warp][4 * lane + 1] = a1;
-    part[warp][4 * lane + 2] = a2;
-    part[warp][4 * lane + 3] = a3;
     __syncthreads();
+    if (ring.abort) return;
     if (tid < TB) {
       float sum = 0.0f;
 #pragma unroll
       for (int w = 0; w < 16; ++w) sum += part[w][tid];
-      wv[tid] = (tid < mk) ? yv[k0 + tid] - sum : 0.0f;
+      wv[tid] = (tid < mk) ? yk - sum : 0.0f;
     }
     __syncthreads();
-    {  // x_K[c] = sum_c' Y_K(c', c) w[c'] (column c of Y_K is contiguous): warp per 8 c
+    if (warp < TRSV_WARPS) {  // x_K[c] = sum_c' Y_K(c', c) w[c'] (column c of Y_K is contiguous): warp per 8 c
       const float4 w4 = reinterpret_cast<const float4 *>(wv)[lane];
       float v[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q)
-        v[q] = warp_sum(ycol[q].x * w4.x + ycol[q].y * w4.y + ycol[q].z * w4.z + ycol[q].w * w4.w);
-      if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (8 * warp + q < mk) __stcg(x + k0 + 8 * warp + q, v[q]);
-        __threadfence();
+        v[q] = ycol[q].x * w4.x + ycol[q].y * w4.y + ycol[q].z * w4.z + ycol[q].w * w4.w;
+      int q;
+      const float xc = warp_sum8(v, q);
+      const int c = 8 * warp + q;
+      if ((lane & 3) == 0) {
+        trsv_put(xp + k0 + c, c < mk ? xc : 0.0f, epoch);
+        if (c < mk) {
+          if (x) x[k0 + c] = xc;
+          if (x64 && k0 + c < n_real) x64[k0 + c] += (double)xc;
+        }
       }
     }
-    __syncthreads();
-    if (tid == 0) st_release_u32(sy.flags + K, epoch);
   }
 }
 
@@ -1150,14 +1275,17 @@ static int chol_blocked_on(RecChol &R, float *A, int64_t lda, int64_t n) {
 // ws[n_tiles][n] is written exactly once; the second kernel sums the slots in
 // a fixed order.
 //
-// GB300 issues about 1.4 FP64 instructions per clock per SM, so a plain FP64
-// symv is bound by the FP64 pipe (~0.6 ms at n = 16,384 even with two FMAs per
-// element) rather than by HBM.  Here each double is split into a (hi, lo) pair
-// of floats with integer operations only and the products are accumulated in
-// double-float arithmetic (~2^-46 relative per term) on the FP32 pipe, which
-// leaves the kernel HBM-bound: n(n+1)/2 * 8 bytes per call.
+// GB300 issues two FP64 operations per clock and SM, so a plain FP64 symv is bound by
+// the FP64 pipe (0.5 ms at n = 16,384 even with two FMAs per element) rather than by
+// HBM.  Here each double is split into a (hi, lo) pair of floats with integer
+// operations only and the products are accumulated in double-float arithmetic
+// (~2^-46 relative per term) on the FP32 pipe.  The all-FP64 solve, whose accuracy
+// must match a direct FP64 factorisation, takes the same tiles in FP64.  (The order of
+// these sums is part of a mixed solution: the residual's last bits move it by 1e-8.)
 constexpr int SY_T = 64;
 constexpr int SY_LD = SY_T + 1;  // smem row stride (floats): conflict-free rows and columns
+
+static int64_t sy_tiles(int64_t n) { return (n + SY_T - 1) / SY_T; }
 
 __device__ inline void sy_tri_tile(int64_t bid, int64_t &I, int64_t &J) {
   int64_t i = (int64_t)((sqrt(8.0 * (double)bid + 1.0) - 1.0) * 0.5);
@@ -1185,6 +1313,18 @@ __device__ __forceinline__ df32 df_split_bits(double a) {
                    __uint_as_float(0x1F800000u);
   return {hi, __uint_as_float(__float_as_uint(lo) | sign)};
 }
+// The same split for 2^-70 <= |a| < 2^127 (df_split_key(a) < DF_SPLIT_KEYS), where neither
+// part leaves the normal range.
+__device__ __forceinline__ uint32_t df_split_key(double a) {
+  return ((uint32_t)__double2hiint(a) & 0x7ff00000u) - 0x3b900000u;
+}
+constexpr uint32_t DF_SPLIT_KEYS = 0x0c500000u;
+__device__ __forceinline__ df32 df_split_normal(double a) {
+  const uint32_t h = (uint32_t)__double2hiint(a), l = (uint32_t)__double2loint(a);
+  const uint32_t f = ((__funnelshift_l(l, h, 3) ^ 0x40000000u) & 0x7fffffffu) | (h & 0x80000000u);
+  const float scale = __uint_as_float((f & 0xff800000u) - (52u << 23));  // sign 2^(e - 52)
+  return {__uint_as_float(f), __uint2float_rz(l & 0x1fffffffu) * scale};
+}
 
 // acc += a * x for double-float a, x (the lo * lo term is below the pair's precision)
 __device__ __forceinline__ df32 df_fma(df32 acc, df32 a, df32 x) {
@@ -1193,151 +1333,256 @@ __device__ __forceinline__ df32 df_fma(df32 acc, df32 a, df32 x) {
   return df_add(acc, p);
 }
 
-__global__ void __launch_bounds__(256) symv_lower_partial_kernel(const double *__restrict__ A,
-                                                                 int64_t n,
-                                                                 const double *__restrict__ x,
-                                                                 double *__restrict__ ws,
-                                                                 const int *done) {
-  if (refine_done(done)) return;
-  __shared__ float ahi[SY_T * SY_LD], alo[SY_T * SY_LD];
-  __shared__ df32 xr[SY_T], xc[SY_T];
-  __shared__ df32 part[4][SY_T];  // [row half 0, row half 1, col half 0, col half 1]
-  int64_t I, J;
-  sy_tri_tile(blockIdx.x, I, J);
-  const int tid = threadIdx.x;
-  const int64_t r0 = I * SY_T, c0 = J * SY_T;
-  const bool diag = (I == J);
-  if (tid < SY_T) xc[tid] = (c0 + tid < n) ? df_split_bits(x[c0 + tid]) : df32{0.0f, 0.0f};
-  else if (tid < 2 * SY_T)
-    xr[tid - SY_T] = (r0 + tid - SY_T < n) ? df_split_bits(x[r0 + tid - SY_T]) : df32{0.0f, 0.0f};
-  {
-    const int c = tid & 63, g = tid >> 6;
-    const bool cok = (c0 + c) < n;
-#pragma unroll 4
-    for (int k = 0; k < 16; ++k) {
-      const int r = g + 4 * k;
-      df32 v{0.0f, 0.0f};
-      if (cok && (r0 + r) < n && (!diag || r >= c)) v = df_split_bits(A[(r0 + r) * n + c0 + c]);
-      ahi[r * SY_LD + c] = v.hi;
-      alo[r * SY_LD + c] = v.lo;
-    }
+template <bool EXACT>
+struct SyNum;
+template <>
+struct SyNum<false> {
+  using V = df32;
+  static __device__ __forceinline__ V zero() { return {0.0f, 0.0f}; }
+  static __device__ __forceinline__ V from(double a) { return df_split_bits(a); }
+  // from() of 16 values none of which needs its rare cases
+  static __device__ __forceinline__ bool plain(const double (&v)[16]) {
+    uint32_t k = 0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) k = max(k, df_split_key(v[i]));
+    return k < DF_SPLIT_KEYS;
   }
-  __syncthreads();
-  // threads 0-127: row sums (row = tid & 63, column half = tid >> 6);
-  // threads 128-255: column sums over the strict lower part of a diagonal tile
-  const int u = tid & 63, h = (tid >> 6) & 1;
-  df32 acc{0.0f, 0.0f};
-  if (tid < 128) {
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) {
-      const int c = 32 * h + i;
-      acc = df_fma(acc, df32{ahi[u * SY_LD + c], alo[u * SY_LD + c]}, xc[c]);
-    }
-  } else {
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) {
-      const int r = 32 * h + i;
-      if (diag && r == u) continue;
-      acc = df_fma(acc, df32{ahi[r * SY_LD + u], alo[r * SY_LD + u]}, xr[r]);
-    }
-  }
-  part[tid >> 6][u] = acc;
-  __syncthreads();
-  if (tid < SY_T) {
-    const int r = tid;
-    const df32 rs = df_add(part[0][r], part[1][r]);
-    const df32 cs = df_add(part[2][r], part[3][r]);
-    if (diag) {
-      if (r0 + r < n) ws[I * n + r0 + r] = df_to_double(df_add(rs, cs));
-    } else {
-      if (r0 + r < n) ws[J * n + r0 + r] = df_to_double(rs);
-      if (c0 + r < n) ws[I * n + c0 + r] = df_to_double(cs);
-    }
-  }
-}
+  static __device__ __forceinline__ V from_plain(double a) { return df_split_normal(a); }
+  static __device__ __forceinline__ V fma(V acc, V a, V x) { return df_fma(acc, a, x); }
+  static __device__ __forceinline__ V add(V a, V b) { return df_add(a, b); }
+  static __device__ __forceinline__ double to(V a) { return df_to_double(a); }
+};
+template <>
+struct SyNum<true> {
+  using V = double;
+  static __device__ __forceinline__ V zero() { return 0.0; }
+  static __device__ __forceinline__ V from(double a) { return a; }
+  static __device__ __forceinline__ bool plain(const double (&)[16]) { return true; }
+  static __device__ __forceinline__ V from_plain(double a) { return a; }
+  static __device__ __forceinline__ V fma(V acc, V a, V x) { return ::fma(a, x, acc); }
+  static __device__ __forceinline__ V add(V a, V b) { return a + b; }
+  static __device__ __forceinline__ double to(V a) { return a; }
+};
 
-__global__ void symv_residual_reduce_kernel(const double *__restrict__ ws, int64_t n, int nt,
-                                            const double *__restrict__ b, double *__restrict__ r,
-                                            const int *done) {
-  if (refine_done(done)) return;
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double s = 0.0;
-  for (int k = 0; k < nt; ++k) s += ws[k * n + i];
-  r[i] = b[i] - s;
-}
+// A CTA walks over the tiles.  Thread (u, h) reads column u of rows 32 h .. 32 h + 31,
+// sixteen rows at a time and sixteen ahead, adds its half of the column's sum straight
+// from the registers, and leaves the elements in shared memory, from where it adds half
+// of row u's.  Bound by the issue of the double-float arithmetic (60 instructions
+// per element).  n = 16,384: 410 -> 310 us, and the launches after convergence 66 -> 2 us
+// each; FP64 at n = 4,096: 46 -> 42 us.
+constexpr int SY_THREADS = 128, SY_CTAS = 5;
 
-// The same tiling in plain FP64 arithmetic (FP64-pipe-bound): the residual of
-// the all-FP64 solve, whose accuracy must match a direct FP64 factorisation.
-__global__ void __launch_bounds__(256) symv_lower_partial_f64_kernel(
-    const double *__restrict__ A, int64_t n, const double *__restrict__ x,
+template <bool EXACT>
+__global__ void __launch_bounds__(SY_THREADS, SY_CTAS) symv_lower_partial_kernel(
+    const double *__restrict__ A, int64_t n, int64_t tiles, const double *__restrict__ x,
     double *__restrict__ ws, const int *done) {
+  using N = SyNum<EXACT>;
+  using V = typename N::V;
   if (refine_done(done)) return;
-  __shared__ double as[SY_T * SY_LD];
-  __shared__ double xr[SY_T], xc[SY_T];
-  __shared__ double part[4][SY_T];
+  __shared__ V as[SY_T * SY_LD];
+  __shared__ V xr[SY_T], xc[SY_T];
+  __shared__ V part[2][2][SY_T];  // [row or column sums][half]
+  const int tid = threadIdx.x, u = tid & 63, h = tid >> 6;
   int64_t I, J;
-  sy_tri_tile(blockIdx.x, I, J);
-  const int tid = threadIdx.x;
-  const int64_t r0 = I * SY_T, c0 = J * SY_T;
-  const bool diag = (I == J);
-  if (tid < SY_T) xc[tid] = (c0 + tid < n) ? x[c0 + tid] : 0.0;
-  else if (tid < 2 * SY_T) xr[tid - SY_T] = (r0 + tid - SY_T < n) ? x[r0 + tid - SY_T] : 0.0;
-  {
-    const int c = tid & 63, g = tid >> 6;
-    const bool cok = (c0 + c) < n;
-#pragma unroll 4
-    for (int k = 0; k < 16; ++k) {
-      const int r = g + 4 * k;
-      double v = 0.0;
-      if (cok && (r0 + r) < n && (!diag || r >= c)) v = A[(r0 + r) * n + c0 + c];
-      as[r * SY_LD + c] = v;
-    }
-  }
-  __syncthreads();
-  const int u = tid & 63, h = (tid >> 6) & 1;
-  double acc = 0.0;
-  if (tid < 128) {
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) {
-      const int c = 32 * h + i;
-      acc = fma(as[u * SY_LD + c], xc[c], acc);
-    }
-  } else {
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) {
-      const int r = 32 * h + i;
-      if (diag && r == u) continue;
-      acc = fma(as[r * SY_LD + u], xr[r], acc);
-    }
-  }
-  part[tid >> 6][u] = acc;
-  __syncthreads();
-  if (tid < SY_T) {
-    const int r = tid;
-    const double rs = part[0][r] + part[1][r];
-    const double cs = part[2][r] + part[3][r];
-    if (diag) {
-      if (r0 + r < n) ws[I * n + r0 + r] = rs + cs;
+  auto load = [&](int q, double (&v)[16]) {
+    const int64_t r0 = I * SY_T + 32 * h + 16 * q, c = J * SY_T + u;
+    const double *p = A + r0 * n + c;
+    if (I != J && (I + 1) * SY_T <= n) {  // J < I: the columns are all there
+#pragma unroll
+      for (int i = 0; i < 16; ++i, p += n) v[i] = __ldg(p);
     } else {
-      if (r0 + r < n) ws[J * n + r0 + r] = rs;
-      if (c0 + r < n) ws[I * n + c0 + r] = cs;
+      const int end = c < n ? (int)(n - r0 < 16 ? n - r0 : 16) : 0;
+      const int first = I == J ? (int)(c - r0) : 0;
+#pragma unroll
+      for (int i = 0; i < 16; ++i, p += n) v[i] = (i < end && i >= first) ? __ldg(p) : 0.0;
+    }
+  };
+  auto load_x = [&]() {
+    const int64_t i = (h ? I : J) * SY_T + u;
+    return i < n ? __ldg(x + i) : 0.0;
+  };
+  double a0[16], a1[16];
+  int64_t t = blockIdx.x;
+  sy_tri_tile(t, I, J);
+  load(0, a0);
+  double xv = load_x();
+  while (true) {
+    load(1, a1);
+    (h ? xr : xc)[u] = N::from(xv);
+    __syncthreads();
+    const bool diag = I == J;
+    V acc = N::zero();
+    auto column = [&](int q, const double (&v)[16]) {
+      const int rq = 32 * h + 16 * q;
+      if (!diag && N::plain(v)) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const V e = N::from_plain(v[i]);
+          as[(rq + i) * SY_LD + u] = e;
+          acc = N::fma(acc, e, xr[rq + i]);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) as[(rq + i) * SY_LD + u] = N::from(v[i]);
+#pragma unroll 1
+        for (int r = rq; r < rq + 16; ++r)
+          if (!(diag && r == u)) acc = N::fma(acc, as[r * SY_LD + u], xr[r]);
+      }
+    };
+    column(0, a0);
+    const int64_t r0 = I * SY_T, c0 = J * SY_T, slot_r = J, slot_c = I;
+    t += gridDim.x;
+    if (t < tiles) {
+      sy_tri_tile(t, I, J);
+      load(0, a0);
+      xv = load_x();
+    }
+    column(1, a1);
+    part[1][h][u] = acc;
+    __syncthreads();
+    acc = N::zero();
+#pragma unroll 8
+    for (int i = 0; i < 32; ++i) acc = N::fma(acc, as[u * SY_LD + 32 * h + i], xc[32 * h + i]);
+    part[0][h][u] = acc;
+    __syncthreads();
+    if (tid < SY_T) {
+      const V rs = N::add(part[0][0][u], part[0][1][u]);
+      const V cs = N::add(part[1][0][u], part[1][1][u]);
+      if (diag) {
+        if (r0 + u < n) ws[slot_c * n + r0 + u] = N::to(N::add(rs, cs));
+      } else {
+        if (r0 + u < n) ws[slot_r * n + r0 + u] = N::to(rs);
+        if (c0 + u < n) ws[slot_c * n + c0 + u] = N::to(cs);
+      }
+    }
+    if (t >= tiles) return;
+  }
+}
+
+// (A x)_i of a block's 32 rows from the nt slots, added in slot order by the first
+// warp; all eight warps load (one warp per row's chain of loads alone took 64 us at
+// n = 16,384, 26 us so).  Valid in warp 0.
+constexpr int SY_ROWS = 32, SY_RED_THREADS = 256, SY_CHUNK = 128;
+
+__device__ __forceinline__ double symv_slots(const double *__restrict__ ws, int64_t n, int64_t nt,
+                                             int64_t i) {
+  __shared__ double sh[SY_CHUNK][SY_ROWS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int PER = SY_CHUNK / (SY_RED_THREADS / 32);
+  double s = 0.0;
+  for (int64_t k0 = 0; k0 < nt; k0 += SY_CHUNK) {
+    double v[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int64_t k = k0 + w * PER + j;
+      v[j] = (k < nt && i < n) ? __ldcg(ws + k * n + i) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < PER; ++j) sh[w * PER + j][lane] = v[j];
+    __syncthreads();
+    const int m = nt - k0 < SY_CHUNK ? (int)(nt - k0) : SY_CHUNK;
+    if (w == 0)
+#pragma unroll 16
+      for (int k = 0; k < m; ++k) s += sh[k][lane];
+    __syncthreads();
+  }
+  return s;
+}
+
+__global__ void __launch_bounds__(SY_RED_THREADS) symv_residual_reduce_kernel(
+    const double *__restrict__ ws, int64_t n, int64_t nt, const double *__restrict__ b,
+    double *__restrict__ r, const int *done) {
+  if (refine_done(done)) return;
+  const int64_t i = blockIdx.x * (int64_t)SY_ROWS + (threadIdx.x & 31);
+  const double s = symv_slots(ws, n, nt, i);
+  if (threadIdx.x < 32 && i < n) r[i] = b[i] - s;
+}
+
+// The slots' sum, r = b - A x, and what the refinement loop asks of it, in one launch:
+// norms = {||r||, ||b||} (each block's sums of squares, added in block order by the
+// last block to finish) and *done as refine_converged_kernel sets it.
+__global__ void __launch_bounds__(SY_RED_THREADS) symv_residual_check_kernel(
+    const double *__restrict__ ws, int64_t n, int64_t nt, const double *__restrict__ b,
+    double *__restrict__ r, double *__restrict__ part, unsigned *counter, double tol,
+    double *norms, double *prev, int *done) {
+  if (refine_done(done)) return;
+  constexpr int WARPS = SY_RED_THREADS / 32;
+  __shared__ double red[2][WARPS];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t i = blockIdx.x * (int64_t)SY_ROWS + lane;
+  const double s = symv_slots(ws, n, nt, i);
+  double sr = 0.0, sb = 0.0;
+  if (w == 0 && i < n) {
+    const double bi = b[i], ri = bi - s;
+    r[i] = ri;
+    sr = ri * ri;
+    sb = bi * bi;
+  }
+  auto both = [&]() {  // block sums of (sr, sb) on thread 0
+    sr = warp_sum(sr);
+    sb = warp_sum(sb);
+    __syncthreads();
+    if (lane == 0) {
+      red[0][w] = sr;
+      red[1][w] = sb;
+    }
+    __syncthreads();
+    sr = sb = 0.0;
+    if (threadIdx.x == 0)
+      for (int k = 0; k < WARPS; ++k) {
+        sr += red[0][k];
+        sb += red[1][k];
+      }
+  };
+  both();
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = sr;
+    part[2 * blockIdx.x + 1] = sb;
+    __threadfence();
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  sr = sb = 0.0;
+  for (int k = threadIdx.x; k < (int)gridDim.x; k += blockDim.x) {
+    sr += __ldcg(part + 2 * k);
+    sb += __ldcg(part + 2 * k + 1);
+  }
+  both();
+  if (threadIdx.x == 0) {
+    *counter = 0u;
+    const double nr = sqrt(sr), nbv = sqrt(sb);
+    norms[0] = nr;
+    norms[1] = nbv;
+    if (nr <= tol * nbv) *done = 1;  // false for NaN: the loop goes on
+    if (prev) {
+      if (nr > 0.5 * *prev) *done = 1;
+      *prev = nr;
     }
   }
+}
+
+static int symv_partial(cudaStream_t st, const double *A, int64_t n, const double *x, double *ws,
+                        const int *done, bool exact) {
+  const int64_t nt = sy_tiles(n), tiles = nt * (nt + 1) / 2;
+  // (one CTA per tile costs 66 us at n = 16,384 in a launch that has nothing to do)
+  const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)SY_CTAS * num_sms());
+  if (exact)
+    symv_lower_partial_kernel<true><<<grid, SY_THREADS, 0, st>>>(A, n, tiles, x, ws, done);
+  else
+    symv_lower_partial_kernel<false><<<grid, SY_THREADS, 0, st>>>(A, n, tiles, x, ws, done);
+  return check_launch("symv partial");
 }
 
 static int symv_residual(cudaStream_t st, const double *A, int64_t n, const double *x,
                          const double *b, double *r, double *ws, const int *done,
                          bool exact = false) {
-  const int64_t nt = (n + SY_T - 1) / SY_T;
-  if (exact)
-    symv_lower_partial_f64_kernel<<<(unsigned)(nt * (nt + 1) / 2), 256, 0, st>>>(A, n, x, ws,
-                                                                                 done);
-  else
-    symv_lower_partial_kernel<<<(unsigned)(nt * (nt + 1) / 2), 256, 0, st>>>(A, n, x, ws, done);
-  int rc = check_launch("symv partial");
+  const int rc = symv_partial(st, A, n, x, ws, done, exact);
   if (rc) return rc;
-  symv_residual_reduce_kernel<<<ceil_div(n, 256), 256, 0, st>>>(ws, n, (int)nt, b, r, done);
+  symv_residual_reduce_kernel<<<ceil_div(n, SY_ROWS), SY_RED_THREADS, 0, st>>>(ws, n, sy_tiles(n),
+                                                                               b, r, done);
   return check_launch("symv reduce");
 }
 
@@ -1463,19 +1708,22 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
   const int64_t np = factor_mode == 4 ? ((n + 3) & ~int64_t(3)) : n;
   const bool own_trsv = (factor_mode == 3 && n % 4 == 0) || factor_mode == 4;
   // aux: r (n double), r32 (np float), two norms + done + prev, symv slots
-  // (n_tiles x n double), inverse diagonal blocks (mode 3), y32 (np float), flags
-  // and tickets (2 nb + 4 uint), leaf inverses (mode 3)
-  const int64_t nt = (n + SY_T - 1) / SY_T;
+  // (strips + segments rows of n double), inverse diagonal blocks (mode 3), the solves' published
+  // words (2 nb TB), tickets and counters (4 uint), residual check partials, leaf
+  // inverses (mode 3)
   const int64_t nb = (np + TB - 1) / TB;
   const size_t r32_off = ((size_t)n * 8 + 255) & ~size_t(255);
   const size_t norms_off = (r32_off + (size_t)np * 4 + 255) & ~size_t(255);
   const size_t ws_off = norms_off + 256;
-  const size_t yinv_off = (ws_off + (size_t)nt * n * 8 + 255) & ~size_t(255);
-  const size_t y32_off =
+  const size_t yinv_off =
+      (ws_off + (size_t)sy_tiles(n) * n * 8 + 255) & ~size_t(255);
+  const size_t words_off =
       (yinv_off + (factor_mode == 3 && own_trsv ? (size_t)nb * TB * TB * 4 : 0) + 255) &
       ~size_t(255);
-  const size_t sync_off = (y32_off + (own_trsv ? (size_t)np * 4 : 0) + 255) & ~size_t(255);
-  const size_t dinv_off = (sync_off + (own_trsv ? (size_t)(2 * nb + 4) * 4 : 0) + 255) & ~size_t(255);
+  const size_t sync_off = words_off + (own_trsv ? (size_t)2 * nb * TB * 8 : 0);
+  const size_t part_off = sync_off + 256;
+  const int check_blocks = ceil_div(n, SY_ROWS);
+  const size_t dinv_off = (part_off + (size_t)check_blocks * 16 + 255) & ~size_t(255);
   const size_t pcg_off = (dinv_off + (factor_mode == 3 ? (size_t)nb * 4096 * 4 : 0) + 255) &
                         ~size_t(255);
   const size_t vec_bytes = ((size_t)n * 8 + 255) & ~size_t(255);
@@ -1489,10 +1737,12 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
   int *done = reinterpret_cast<int *>(norms + 3);
   double *sws = reinterpret_cast<double *>(aux + ws_off);
   float *yinv = reinterpret_cast<float *>(aux + yinv_off);
-  float *y32 = reinterpret_cast<float *>(aux + y32_off);
-  unsigned *sync = reinterpret_cast<unsigned *>(aux + sync_off);
-  const TrsvSync sync_f{sync, sync + 2 * nb, sync + 2 * nb + 2, wait_limit_ns()};
-  const TrsvSync sync_b{sync + nb, sync + 2 * nb + 1, sync + 2 * nb + 2, wait_limit_ns()};
+  unsigned long long *yp = reinterpret_cast<unsigned long long *>(aux + words_off);
+  unsigned long long *xp = yp + nb * TB;
+  unsigned *sync = reinterpret_cast<unsigned *>(aux + sync_off);  // tickets, abort, counter
+  const TrsvSync sync_f{sync, sync + 1, sync + 2, wait_limit_ns()};
+  const TrsvSync sync_b{sync + 1, sync, sync + 2, wait_limit_ns()};
+  double *check_part = reinterpret_cast<double *>(aux + part_off);
   float *F = A32;  // the factor the solves read
   if (factor_mode == 4) {
     const size_t pad_bytes = np != n ? (size_t)np * np * 4 : 0;
@@ -1513,7 +1763,6 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
     if (np != n)
       VMCK_CUDA(cudaMemcpy2DAsync(A32, n * 4, F, np * 4, n * 4, n, cudaMemcpyDeviceToDevice, st));
     VMCK_CUDA(cudaMemsetAsync(c->d_info, 0, sizeof(int), st));
-    VMCK_CUDA(cudaMemsetAsync(sync, 0, (size_t)(2 * nb + 4) * 4, st));
   } else if (factor_mode >= 2) {
     VMCK_BLAS(cublasSetMathMode(c->blas, CUBLAS_FP32_EMULATED_BF16X9_MATH));
     VMCK_BLAS(cublasSetEmulationStrategy(c->blas, CUBLAS_EMULATION_STRATEGY_EAGER));
@@ -1545,7 +1794,6 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
                                      (int)TRSM_SMEM));
       trsv_inv_kernel<<<dim3(2, (unsigned)nb), LEAF_THREADS, TRSM_SMEM, st>>>(A32, n, yinv);
       if ((rc = check_launch("refined solve inverse blocks"))) return rc;
-      VMCK_CUDA(cudaMemsetAsync(sync, 0, (size_t)(2 * nb + 4) * 4, st));
     }
   } else {
     cusolverStatus_t fs = cusolverDnXpotrf(c->solver, c->params, CUBLAS_FILL_MODE_UPPER, n,
@@ -1559,6 +1807,11 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
     info_accumulate_kernel<<<1, 1, 0, st>>>(c->d_info, status);
     if ((rc = check_launch("refined solve info"))) return rc;
   }
+  if (own_trsv)
+    VMCK_CUDA(cudaFuncSetAttribute(trsv_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)TRSV_SMEM));
+  // no published words, tickets at 0 (words and sync are adjacent)
+  VMCK_CUDA(cudaMemsetAsync(yp, 0, part_off - words_off, st));
   if (o.pcg) {
     VMCK_REQUIRE(own_trsv, "the PCG fallback runs on the tensor-core factor (factor_mode 4)");
     // a failed factor is reported before any iteration: the caller retries with
@@ -1582,20 +1835,16 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
     VMCK_CUDA(cudaMemcpyAsync(r, b, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
     refine_init_kernel<<<1, 32, 0, st>>>(norms, prev, done);
     if ((rc = check_launch("pcg init"))) return rc;
-    if (np != n) VMCK_CUDA(cudaMemsetAsync(r32, 0, (size_t)np * 4, st));
     unsigned epoch = 0;
     // z = M^-1 r: the two triangular solves on the factor of A32
     auto precondition = [&]() -> int {
       int e;
-      d2f_kernel<<<blocks, 256, 0, st>>>(r, r32, n, done);
-      if ((e = check_launch("pcg cast"))) return e;
       ++epoch;
-      VMCK_CUDA(cudaMemsetAsync(sync + 2 * nb, 0, 2 * sizeof(unsigned), st));  // tickets
-      trsv_fwd_kernel<<<grid, LEAF_THREADS, 0, st>>>(F, np, yinv, r32, y32, sync_f, epoch,
-                                                     status, done);
+      trsv_fwd_kernel<<<grid, TRSV_THREADS, TRSV_SMEM, st>>>(F, np, yinv, r, n, yp, sync_f, epoch, status,
+                                                     done);
       if ((e = check_launch("pcg forward"))) return e;
-      trsv_bwd_kernel<<<grid, LEAF_THREADS, 0, st>>>(F, np, yinv, y32, r32, sync_b, epoch,
-                                                     status, done);
+      trsv_bwd_kernel<<<grid, TRSV_THREADS, 0, st>>>(F, np, yinv, yp, xp, r32, nullptr, n, sync_b,
+                                                     epoch, status, done);
       if ((e = check_launch("pcg backward"))) return e;
       f2d_copy_kernel<<<blocks, 256, 0, st>>>(r32, z, n, done);
       return check_launch("pcg z");
@@ -1643,41 +1892,41 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
   VMCK_CUDA(cudaMemsetAsync(x, 0, (size_t)n * 8, st));
   refine_init_kernel<<<1, 32, 0, st>>>(norms, prev, done);  // norms 0, prev huge, done 0
   if ((rc = check_launch("refined solve init"))) return rc;
-  if (np != n) VMCK_CUDA(cudaMemsetAsync(r32, 0, (size_t)np * 4, st));
-  const int blocks = ceil_div(n, 256);
+  // r = b - A x, its norm and whether the loop is done
+  auto residual = [&]() -> int {
+    int e = symv_partial(st, A64, n, x, sws, done, o.exact);
+    if (e) return e;
+    symv_residual_check_kernel<<<check_blocks, SY_RED_THREADS, 0, st>>>(
+        sws, n, sy_tiles(n), b, r, check_part, sync + 3, o.stop_tol, norms,
+        o.stagnation ? prev : nullptr, done);
+    return check_launch("refined solve residual");
+  };
+  const unsigned grid = (unsigned)std::min<int64_t>(nb, 2 * (int64_t)num_sms());
   // Iteration it > 0 first forms r = b - A x and stops the loop (on the device)
-  // once it is small enough; the kernels after that return at entry.
+  // once it is small enough; the kernels after that return at entry.  (Four
+  // launches per iteration: with up to 30 of them in the FP64 solve, most of which
+  // find the loop done, each costs about 2 us.)
   for (int it = 0; it < o.max_iter; ++it) {
-    if (it == 0) {
-      VMCK_CUDA(cudaMemcpyAsync(r, b, (size_t)n * 8, cudaMemcpyDeviceToDevice, st));
-    } else {
-      if ((rc = symv_residual(st, A64, n, x, b, r, sws, done, o.exact))) return rc;
-      refine_converged_kernel<<<1, 256, 0, st>>>(r, b, n, o.stop_tol, done,
-                                                 o.stagnation ? prev : nullptr);
-      if ((rc = check_launch("refined solve convergence"))) return rc;
-    }
-    d2f_kernel<<<blocks, 256, 0, st>>>(r, r32, n, done);
-    if ((rc = check_launch("refined solve cast"))) return rc;
+    if (it > 0 && (rc = residual())) return rc;
+    const double *rhs = it == 0 ? b : r;
     if (own_trsv) {
-      const unsigned grid = (unsigned)std::min<int64_t>(nb, 2 * (int64_t)num_sms());
-      VMCK_CUDA(cudaMemsetAsync(sync + 2 * nb, 0, 2 * sizeof(unsigned), st));  // tickets
-      trsv_fwd_kernel<<<grid, LEAF_THREADS, 0, st>>>(F, np, yinv, r32, y32, sync_f,
+      trsv_fwd_kernel<<<grid, TRSV_THREADS, TRSV_SMEM, st>>>(F, np, yinv, rhs, n, yp, sync_f,
                                                      (unsigned)(it + 1), status, done);
       if ((rc = check_launch("refined solve forward"))) return rc;
-      trsv_bwd_kernel<<<grid, LEAF_THREADS, 0, st>>>(F, np, yinv, y32, r32, sync_b,
+      trsv_bwd_kernel<<<grid, TRSV_THREADS, 0, st>>>(F, np, yinv, yp, xp, nullptr, x, n, sync_b,
                                                      (unsigned)(it + 1), status, done);
       if ((rc = check_launch("refined solve backward"))) return rc;
     } else {
+      d2f_kernel<<<ceil_div(n, 256), 256, 0, st>>>(rhs, r32, n, done);
+      if ((rc = check_launch("refined solve cast"))) return rc;
       VMCK_SOLVER(cusolverDnXpotrs(c->solver, c->params, CUBLAS_FILL_MODE_UPPER, n, 1, CUDA_R_32F,
                                    A32, n, CUDA_R_32F, r32, n, c->d_info));
+      axpy_f2d_kernel<<<ceil_div(n, 256), 256, 0, st>>>(x, r32, n, done);
+      if ((rc = check_launch("refined solve update"))) return rc;
     }
-    axpy_f2d_kernel<<<blocks, 256, 0, st>>>(x, r32, n, done);
-    if ((rc = check_launch("refined solve update"))) return rc;
   }
   // the final residual (skipped when the loop stopped early: r already belongs to x)
-  if ((rc = symv_residual(st, A64, n, x, b, r, sws, done, o.exact))) return rc;
-  norms_kernel<<<1, 256, 0, st>>>(r, b, n, norms);
-  if ((rc = check_launch("refined solve norms"))) return rc;
+  if ((rc = residual())) return rc;
   refine_check_kernel<<<1, 1, 0, st>>>(norms, norms + 1, c->d_info, o.fail_tol, status,
                                        residual_out);
   return check_launch("refined solve");
