@@ -196,10 +196,10 @@ int vmck_rbm_eloc_local(vmck_stream s, int32_t dtype, const void *params, int32_
                         int32_t M, const int8_t *x, int64_t n, const vmck_local_op *op,
                         double *eloc, void *logpsi_out);
 /* The same in FP64 from tables of flip factors exp(+-4 W), made once per call in
- * the caller's workspace (at least vmck_rbm_eloc_f64_workspace_size(N, M)
- * doubles): a few FP64 operations per hidden unit and connected element instead
- * of a log_cosh. */
-int64_t vmck_rbm_eloc_f64_workspace_size(int32_t N, int32_t M);
+ * the caller's workspace (at least vmck_rbm_eloc_f64_workspace_size(N, M, n)
+ * doubles): one factor per hidden unit and connected element, in 64-bit fixed point
+ * for flips of one or two sites, instead of a log_cosh. */
+int64_t vmck_rbm_eloc_f64_workspace_size(int32_t N, int32_t M, int64_t n);
 int vmck_rbm_eloc_ising_f64(vmck_stream s, const double *params, int32_t N, int32_t M,
                             const int8_t *x, int64_t n, const int32_t *edges,
                             int32_t n_edges, double h, double J, double *eloc,

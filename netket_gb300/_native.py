@@ -91,7 +91,7 @@ _SIGNATURES = {
                              c_dbl, c_vp, c_vp], c_i32),
     "vmck_rbm_eloc_local": ([c_vp, c_i32, c_vp, c_i32, c_i32, c_vp, c_i64,
                              ctypes.POINTER(LocalOpStruct), c_vp, c_vp], c_i32),
-    "vmck_rbm_eloc_f64_workspace_size": ([c_i32, c_i32], c_i64),
+    "vmck_rbm_eloc_f64_workspace_size": ([c_i32, c_i32, c_i64], c_i64),
     "vmck_rbm_eloc_ising_f64": ([c_vp, c_vp, c_i32, c_i32, c_vp, c_i64, c_vp, c_i32, c_dbl, c_dbl,
                                  c_vp, c_vp, c_i64], c_i32),
     "vmck_rbm_eloc_local_f64": ([c_vp, c_vp, c_i32, c_i32, c_vp, c_i64,

@@ -1,7 +1,7 @@
 // FP64 products with the spin matrix by tables of signed sums (signsum_f64.cu).
 #pragma once
 
-#include "common.cuh"
+#include "units_f64.cuh"
 
 namespace vmck {
 
@@ -10,6 +10,9 @@ namespace vmck {
 bool signed_rows_fit(int N);
 int logpsi_f64(cudaStream_t st, const double *params, int N, int M, const int8_t *x, int64_t n,
                double *logpsi, double *theta, double *tanh_out);
+// theta and q_units(theta) of n samples
+int theta_q_f64(cudaStream_t st, const double *params, int N, int M, const int8_t *x, int64_t n,
+                double *theta, u64 *q);
 // out_s = t_s . (v_bias + x_s V) + x_s . v_visible
 int o_v_f64(cudaStream_t st, const double *t, const int8_t *x, int N, int M, int64_t n,
             const double *v, double *out);

@@ -18,9 +18,9 @@
 // Lanes are hidden units, so a lookup reads 256 consecutive bytes of shared memory
 // at an address that the warp shares.
 //
-// log_cosh: sum_j log_cosh(theta_j) = sum |theta| + log prod (1 + e^(-2|theta|))
-// - M log 2: a product per hidden unit instead of a log1p; tanh shares the
-// exponential (expm1, so that it keeps its relative precision near 0).
+// log_cosh: sum_j log_cosh(theta_j) = sum |theta| + log prod (1 + e^(-2|theta|)) / 2
+// over a lane's hidden units: a product per hidden unit instead of a log1p; tanh shares
+// the exponential (expm1, so that it keeps its relative precision near 0).
 //
 // O^T v is bound by the issue of the lookups (six instructions each), theta and O v by
 // the barriers around a tile's tables.  Measured (GB300, kernel time; before = tables of
@@ -38,6 +38,8 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "units_f64.cuh"
+
 namespace vmck {
 
 namespace cg = cooperative_groups;
@@ -48,7 +50,8 @@ constexpr int SR_THREADS = 256, SR_WARPS = SR_THREADS / 32;
 constexpr int SS_TAB = 16 * 32;  // entries per group of four
 constexpr int SR_HELD = 4;       // groups of a warp held in registers
 constexpr int SR_BLOCK = 26;     // groups per table block: two CTAs' tables in an SM
-constexpr int SR_SITES_MAX = 2048;
+constexpr int64_t SR_INDEX_MAX = 32 * 1024;  // bytes of sign indices per CTA
+constexpr int SR_SITES_MAX = 16384;
 
 // acc + the table's entry number `byte` (a byte of four, moved to bits 8 to 11: the
 // entries are 256 bytes apart)
@@ -84,53 +87,20 @@ __device__ __forceinline__ void fill_table(T *tab, T w0, T w1, T w2, T w3) {
   tab[15 * 32] = -ps;
 }
 
-// Size of an entry for the largest of a column: the high word without its sign, its
-// last bit set where only the low word is not 0.
-__device__ __forceinline__ uint32_t size_word(double w) {
-  return ((uint32_t)__double2hiint(w) & 0x7fffffffu) | (__double2loint(w) != 0 ? 1u : 0u);
-}
-// Whether entries below 2^(e - 1022) have the integer form
-__device__ __forceinline__ bool exponent_fits(int e) { return e >= 200 && e <= 1900; }
-// w, |w| < 2^(e - 1022), in units of unit_of(e, bits); |result| <= 2^bits
-__device__ __forceinline__ long long to_units(double w, int e, int bits) {
-  const int hi = __double2hiint(w), ew = (hi >> 20) & 0x7ff;
-  const unsigned long long m =
-      (unsigned long long)(uint32_t)((hi & 0xfffff) | (ew ? 0x100000 : 0)) << 32 |
-      (uint32_t)__double2loint(w);
-  const int s = bits - 53 - (e - (ew ? ew : 1));
-  unsigned long long q = 0ull;
-  if (s >= 0)
-    q = m << s;
-  else if (s > -55)
-    q = (m + (1ull << (-s - 1))) >> -s;
-  return hi < 0 ? -(long long)q : (long long)q;
-}
-__device__ __forceinline__ double unit_of(int e, int bits) {
-  return __hiloint2double((e + 1 - bits) << 20, 0);
-}
-// bits that leave room for a sum of `terms` entries
-__host__ __device__ __forceinline__ int sum_bits(int64_t terms) {
-  int b = 62;
-  while (terms > 1) {
-    terms = (terms + 1) >> 1;
-    --b;
-  }
-  return b;
-}
-
-enum RowsOut { ROWS_LOGPSI = 0, ROWS_DOT = 1 };
+enum RowsOut { ROWS_LOGPSI = 0, ROWS_DOT = 1, ROWS_THETA = 2 };
 
 // A cluster takes SR_WARPS * SPW samples; its CTAs share the tiles of 32 hidden units
 // (a table serves all of the cluster's samples) and the first adds their sums.  Per
 // tile: the tables (4 KB per four sites, `block` groups of sites at a time), then each
 // warp its SPW samples.
 //   ROWS_LOGPSI: out = logpsi, optional theta_out / tanh_out;
-//   ROWS_DOT: out = sum_j t_sj theta_sj + x . a.
+//   ROWS_DOT: out = sum_j t_sj theta_sj + x . a;
+//   ROWS_THETA: theta_out and q_out = q_units(theta).
 template <RowsOut OUT, int SPW>
 __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
     const double *__restrict__ params, const int8_t *__restrict__ x, int N, int M, int64_t n,
     int block, const double *__restrict__ t, double *__restrict__ out,
-    double *__restrict__ theta_out, double *__restrict__ tanh_out) {
+    double *__restrict__ theta_out, double *__restrict__ tanh_out, u64 *__restrict__ q_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t largest[SR_WARPS][32];
   __shared__ double sum[SR_WARPS * SPW];
@@ -161,6 +131,7 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
   const uint8_t *mine = index + (size_t)warp * SPW * G4;
   const int64_t sw = s0 + warp * SPW;  // this warp's first sample
   double acc[SPW], prod[SPW];
+  int units = 0;  // this lane's hidden units
 #pragma unroll
   for (int s = 0; s < SPW; ++s) {
     acc[s] = 0.0;
@@ -178,6 +149,7 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
     const int j = j0 + lane;
     const bool in = j < M;
     const double bj = in ? params[j] : 0.0;
+    units += in;
     uint32_t size = 0u;
 #pragma unroll
     for (int k = 0; k < SR_HELD; ++k)
@@ -259,6 +231,11 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
     for (int s = 0; s < SPW; ++s) {
       const int64_t row = sw + s;
       if (!in || row >= n) continue;
+      if (OUT == ROWS_THETA) {
+        theta_out[row * M + j] = th[s];
+        q_out[row * M + j] = q_units(th[s]);
+        continue;
+      }
       if (OUT == ROWS_DOT) {
         acc[s] = fma(ts[s], th[s], acc[s]);
         continue;
@@ -275,29 +252,31 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
       if (theta_out) theta_out[row * M + j] = th[s];
     }
   }
+  if constexpr (OUT != ROWS_THETA) {
 #pragma unroll
-  for (int s = 0; s < SPW; ++s)  // at most 2^(M / 32) per lane
-    if (OUT == ROWS_LOGPSI) acc[s] += log(prod[s]);
-  if (rank == 0)
-    for (int i = lane; i < N; i += 32) {
-      const double ai = __ldg(a + i);
+    for (int s = 0; s < SPW; ++s)  // at most 2^(M / 32) per lane; log 2 taken out exactly
+      if (OUT == ROWS_LOGPSI) acc[s] += log(ldexp(prod[s], -units));
+    if (rank == 0)
+      for (int i = lane; i < N; i += 32) {
+        const double ai = __ldg(a + i);
 #pragma unroll
-      for (int s = 0; s < SPW; ++s)
-        if (sw + s < n) acc[s] += x[(sw + s) * N + i] < 0 ? -ai : ai;
+        for (int s = 0; s < SPW; ++s)
+          if (sw + s < n) acc[s] += x[(sw + s) * N + i] < 0 ? -ai : ai;
+      }
+#pragma unroll
+    for (int s = 0; s < SPW; ++s) {
+      const double v = warp_sum(acc[s]);
+      if (lane == 0) sum[warp * SPW + s] = v;
     }
-#pragma unroll
-  for (int s = 0; s < SPW; ++s) {
-    const double v = warp_sum(acc[s]);
-    if (lane == 0) sum[warp * SPW + s] = v;
+    if (ranks > 1) cluster.sync();
+    else __syncthreads();
+    if (rank == 0 && tid < SR_WARPS * SPW && s0 + tid < n) {
+      double v = sum[tid];
+      for (int r = 1; r < ranks; ++r) v += cluster.map_shared_rank(sum, r)[tid];
+      out[s0 + tid] = v;
+    }
+    if (ranks > 1) cluster.sync();  // the others' sums stay until they are read
   }
-  if (ranks > 1) cluster.sync();
-  else __syncthreads();
-  if (rank == 0 && tid < SR_WARPS * SPW && s0 + tid < n) {
-    double v = sum[tid];
-    for (int r = 1; r < ranks; ++r) v += cluster.map_shared_rank(sum, r)[tid];
-    out[s0 + tid] = OUT == ROWS_LOGPSI ? v - M * 0.69314718055994530942 : v;
-  }
-  if (ranks > 1) cluster.sync();  // the others' sums stay until they are read
 }
 
 int sm_count() {
@@ -309,7 +288,8 @@ int sm_count() {
 
 template <RowsOut OUT, int SPW>
 int launch_rows_as(cudaStream_t st, int ranks, const double *params, const int8_t *x, int N, int M,
-                   int64_t n, const double *t, double *out, double *theta, double *tanh_out) {
+                   int64_t n, const double *t, double *out, double *theta, double *tanh_out,
+                   u64 *q) {
   const int G = (N + 3) / 4, G4 = (G + 3) & ~3;
   // equal blocks of whole fours (an index word holds four groups)
   const int blocks = G <= SR_BLOCK ? 1 : (G + 23) / 24;
@@ -331,8 +311,8 @@ int launch_rows_as(cudaStream_t st, int ranks, const double *params, const int8_
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   VMCK_CUDA(cudaLaunchKernelEx(&cfg, signed_rows_kernel<OUT, SPW>, params, x, N, M, n, block, t,
-                               out, theta, tanh_out));
-  return check_launch(OUT == ROWS_LOGPSI ? "rbm_logpsi" : "rbm_o_v");
+                               out, theta, tanh_out, q));
+  return check_launch("rows of signed sums");
 }
 
 // Clusters of two: they halve the tables per sample (n = 4,096, N = 100, M = 200 / 400:
@@ -342,16 +322,18 @@ int launch_rows_as(cudaStream_t st, int ranks, const double *params, const int8_
 // (half as many samples each: 50 / 75 us).
 template <RowsOut OUT>
 int launch_rows(cudaStream_t st, const double *params, const int8_t *x, int N, int M, int64_t n,
-                const double *t, double *out, double *theta, double *tanh_out) {
+                const double *t, double *out, double *theta, double *tanh_out, u64 *q) {
   const int ranks = M > 32 ? 2 : 1;
   const int64_t full = (int64_t)sm_count() * SR_WARPS / ranks;
-  if (n >= 8 * full)
-    return launch_rows_as<OUT, 8>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out);
-  if (n >= 4 * full)
-    return launch_rows_as<OUT, 4>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out);
-  if (n >= 2 * full)
-    return launch_rows_as<OUT, 2>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out);
-  return launch_rows_as<OUT, 1>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out);
+  // (very many sites: fewer samples' index bytes, one per four sites)
+  const int64_t per = SR_WARPS * ((N + 15) / 16 * 4);
+  if (n >= 8 * full && 8 * per <= SR_INDEX_MAX)
+    return launch_rows_as<OUT, 8>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out, q);
+  if (n >= 4 * full && 4 * per <= SR_INDEX_MAX)
+    return launch_rows_as<OUT, 4>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out, q);
+  if (n >= 2 * full && 2 * per <= SR_INDEX_MAX)
+    return launch_rows_as<OUT, 2>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out, q);
+  return launch_rows_as<OUT, 1>(st, ranks, params, x, N, M, n, t, out, theta, tanh_out, q);
 }
 
 // ------------------------------------------------------------ O^T v
@@ -511,17 +493,23 @@ int launch_ot_v(cudaStream_t st, dim3 grid, const double *t, const int8_t *x, in
 
 }  // namespace
 
-// (an index byte per four sites of up to 64 samples in shared memory)
+// (an index byte per four sites of eight samples in shared memory)
 bool signed_rows_fit(int N) { return N <= SR_SITES_MAX; }
 
 int logpsi_f64(cudaStream_t st, const double *params, int N, int M, const int8_t *x, int64_t n,
                double *logpsi, double *theta, double *tanh_out) {
-  return launch_rows<ROWS_LOGPSI>(st, params, x, N, M, n, nullptr, logpsi, theta, tanh_out);
+  return launch_rows<ROWS_LOGPSI>(st, params, x, N, M, n, nullptr, logpsi, theta, tanh_out,
+                                  nullptr);
 }
 
 int o_v_f64(cudaStream_t st, const double *t, const int8_t *x, int N, int M, int64_t n,
             const double *v, double *out) {
-  return launch_rows<ROWS_DOT>(st, v, x, N, M, n, t, out, nullptr, nullptr);
+  return launch_rows<ROWS_DOT>(st, v, x, N, M, n, t, out, nullptr, nullptr, nullptr);
+}
+
+int theta_q_f64(cudaStream_t st, const double *params, int N, int M, const int8_t *x, int64_t n,
+                double *theta, u64 *q) {
+  return launch_rows<ROWS_THETA>(st, params, x, N, M, n, nullptr, nullptr, theta, nullptr, q);
 }
 
 int ot_v_f64_chunks(int N, int M, int64_t n) {

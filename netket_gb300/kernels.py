@@ -66,8 +66,8 @@ def local_energies_fused(op, params_c, x, N, M):
                                                 nat.ptr(x), n, ctypes.byref(st), nat.ptr(e), None))
         return e
     if params_c.dtype == torch.float64 and isinstance(op, (Ising, LocalOperator)):
-        ws = torch.empty(nat.lib().vmck_rbm_eloc_f64_workspace_size(N, M), dtype=torch.float64,
-                         device=x.device)
+        ws = torch.empty(nat.lib().vmck_rbm_eloc_f64_workspace_size(N, M, n),
+                         dtype=torch.float64, device=x.device)
         if isinstance(op, Ising):
             nat.check(nat.lib().vmck_rbm_eloc_ising_f64(
                 nat.stream(), nat.ptr(params_c), N, M, nat.ptr(x), n, nat.ptr(op._edges_dev()),
