@@ -1124,6 +1124,12 @@ int chol_tc_factor(cudaStream_t st, float *A, int64_t n, void *ws, int32_t *stat
     if (split) VMCK_CUDA(cudaStreamWaitEvent(ls->chain2, ls->events[3 * nblocks], 0));
   }
   const int side_grid = two ? side_ctas(num_sms_dev(), n) : 0;
+  // chain2's updates leave two of the SMs that the side stream does not use: a grid
+  // over all of them keeps the next leaf waiting for its last wave (n = 16,384: factor
+  // and two refinements 11.87 -> 11.30 ms; 11.75 with none left, 11.36 with four, 11.63
+  // with sixteen; n = 24,000: 27.7 -> 26.35).  Before the first trailing update the
+  // whole chip is the chain's, and a reserve there changes nothing.
+  const int chain2_grid = std::max(8, num_sms_dev() - side_grid - 2);
   VMCK_CUDA(cudaFuncSetAttribute(chol_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)CHOL_LEAF_SMEM));
   // the leaf writes X and Y on and above, or below, their diagonals
@@ -1206,7 +1212,7 @@ int chol_tc_factor(cudaStream_t st, float *A, int64_t n, void *ws, int32_t *stat
             if ((rc = tc_gemm(ls->chain2, pk, (int)(r2 - k0), pk, (int)(r2 - k0), pp * LB,
                               (int)(k1 - r2), (int)(n - r2), mp, A + r2 + r2 * n, n, -1.0f,
                               1.0f, scales + 1, scales + 1, 1, nullptr, nullptr, 0, 0, 0,
-                              nullptr, status, 0)))
+                              nullptr, status, b == 0 ? 0 : chain2_grid)))
               return rc;
             VMCK_CUDA(cudaEventRecord(PB[pi], ls->chain2));
             pb_pending = true;

@@ -888,6 +888,8 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1)
     trsv_fwd_kernel(const float *__restrict__ U, int64_t n, const float *__restrict__ Yinv,
                     const double *__restrict__ r, int64_t n_real, unsigned long long *yp,
                     TrsvSync sy, unsigned epoch, int32_t *status, const int *done) {
+  pdl_wait();
+  pdl_trigger();
   if (refine_done(done)) return;  // before any ticket: every CTA leaves
   extern __shared__ __align__(16) float ysm[];  // Y_K, column-major
   __shared__ TrsvRing ring;
@@ -972,6 +974,8 @@ __global__ void __launch_bounds__(TRSV_THREADS, 1)
                     const unsigned long long *__restrict__ yp, unsigned long long *xp, float *x,
                     double *x64, int64_t n_real, TrsvSync sy, unsigned epoch, int32_t *status,
                     const int *done) {
+  pdl_wait();
+  pdl_trigger();
   if (refine_done(done)) return;
   __shared__ TrsvRing ring;
   __shared__ __align__(16) float wv[TB];
@@ -1267,6 +1271,25 @@ static int chol_blocked_on(RecChol &R, float *A, int64_t lda, int64_t n) {
   return VMCK_OK;
 }
 
+// Launch of one of the refinement loop's kernels, which begin with pdl_wait(): its CTAs
+// may be placed while the previous kernel of the stream still runs.
+template <typename... P, typename... Args>
+static int launch_early(void (*kernel)(P...), unsigned grid, unsigned threads, size_t smem,
+                        cudaStream_t st, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  VMCK_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  return check_launch("refined solve");
+}
+
 // ------------------------------------------------------------ symmetric residual
 // r = b - A x for a symmetric A stored as its lower triangle (row-major), each
 // stored element read exactly once.  Tile (I, J), I >= J, of 64 x 64 adds
@@ -1378,6 +1401,8 @@ __global__ void __launch_bounds__(SY_THREADS, SY_CTAS) symv_lower_partial_kernel
     double *__restrict__ ws, const int *done) {
   using N = SyNum<EXACT>;
   using V = typename N::V;
+  pdl_wait();
+  pdl_trigger();
   if (refine_done(done)) return;
   __shared__ V as[SY_T * SY_LD];
   __shared__ V xr[SY_T], xc[SY_T];
@@ -1505,6 +1530,8 @@ __global__ void __launch_bounds__(SY_RED_THREADS) symv_residual_check_kernel(
     const double *__restrict__ ws, int64_t n, int64_t nt, const double *__restrict__ b,
     double *__restrict__ r, double *__restrict__ part, unsigned *counter, double tol,
     double *norms, double *prev, int *done) {
+  pdl_wait();
+  pdl_trigger();
   if (refine_done(done)) return;
   constexpr int WARPS = SY_RED_THREADS / 32;
   __shared__ double red[2][WARPS];
@@ -1569,11 +1596,8 @@ static int symv_partial(cudaStream_t st, const double *A, int64_t n, const doubl
   const int64_t nt = sy_tiles(n), tiles = nt * (nt + 1) / 2;
   // (one CTA per tile costs 66 us at n = 16,384 in a launch that has nothing to do)
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, (int64_t)SY_CTAS * num_sms());
-  if (exact)
-    symv_lower_partial_kernel<true><<<grid, SY_THREADS, 0, st>>>(A, n, tiles, x, ws, done);
-  else
-    symv_lower_partial_kernel<false><<<grid, SY_THREADS, 0, st>>>(A, n, tiles, x, ws, done);
-  return check_launch("symv partial");
+  return launch_early(exact ? symv_lower_partial_kernel<true> : symv_lower_partial_kernel<false>,
+                      grid, SY_THREADS, 0, st, A, n, tiles, x, ws, done);
 }
 
 static int symv_residual(cudaStream_t st, const double *A, int64_t n, const double *x,
@@ -1896,26 +1920,26 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
   auto residual = [&]() -> int {
     int e = symv_partial(st, A64, n, x, sws, done, o.exact);
     if (e) return e;
-    symv_residual_check_kernel<<<check_blocks, SY_RED_THREADS, 0, st>>>(
-        sws, n, sy_tiles(n), b, r, check_part, sync + 3, o.stop_tol, norms,
-        o.stagnation ? prev : nullptr, done);
-    return check_launch("refined solve residual");
+    return launch_early(symv_residual_check_kernel, check_blocks, SY_RED_THREADS, 0, st, sws, n,
+                        sy_tiles(n), b, r, check_part, sync + 3, o.stop_tol, norms,
+                        o.stagnation ? prev : nullptr, done);
   };
   const unsigned grid = (unsigned)std::min<int64_t>(nb, 2 * (int64_t)num_sms());
   // Iteration it > 0 first forms r = b - A x and stops the loop (on the device)
   // once it is small enough; the kernels after that return at entry.  (Four
-  // launches per iteration: with up to 30 of them in the FP64 solve, most of which
-  // find the loop done, each costs about 2 us.)
+  // launches per iteration, each placed while the one before it runs: with up to 30
+  // of them in the FP64 solve, most of which find the loop done, this takes 0.33 ms
+  // off 3.43 ms at n = 4,096.)
   for (int it = 0; it < o.max_iter; ++it) {
     if (it > 0 && (rc = residual())) return rc;
     const double *rhs = it == 0 ? b : r;
     if (own_trsv) {
-      trsv_fwd_kernel<<<grid, TRSV_THREADS, TRSV_SMEM, st>>>(F, np, yinv, rhs, n, yp, sync_f,
-                                                     (unsigned)(it + 1), status, done);
-      if ((rc = check_launch("refined solve forward"))) return rc;
-      trsv_bwd_kernel<<<grid, TRSV_THREADS, 0, st>>>(F, np, yinv, yp, xp, nullptr, x, n, sync_b,
-                                                     (unsigned)(it + 1), status, done);
-      if ((rc = check_launch("refined solve backward"))) return rc;
+      if ((rc = launch_early(trsv_fwd_kernel, grid, TRSV_THREADS, TRSV_SMEM, st, F, np, yinv, rhs,
+                             n, yp, sync_f, (unsigned)(it + 1), status, done)))
+        return rc;
+      if ((rc = launch_early(trsv_bwd_kernel, grid, TRSV_THREADS, 0, st, F, np, yinv, yp, xp,
+                             nullptr, x, n, sync_b, (unsigned)(it + 1), status, done)))
+        return rc;
     } else {
       d2f_kernel<<<ceil_div(n, 256), 256, 0, st>>>(rhs, r32, n, done);
       if ((rc = check_launch("refined solve cast"))) return rc;
