@@ -18,33 +18,61 @@ __device__ __forceinline__ float ex2_fast(float x) {
   return y;
 }
 
-// The plain kernel's decision in FP64, theta formed from scratch for the spins in
-// the words xb (word l in lane l).
+// theta_j for the spins in the words xb (word l in lane l), from scratch, the sites in
+// order, four loads in flight.  j < 0: this lane has no hidden unit.
+__device__ __forceinline__ double theta_f64(const double *__restrict__ params, int N, int M,
+                                            uint32_t xb, int j) {
+  const double *W = params + M + max(j, 0);
+  double th = __ldg(params + max(j, 0));
+  for (int w = 0; 32 * w < N; ++w) {
+    const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
+    const int i1 = min(32, N - 32 * w);
+    for (int q0 = 0; q0 < i1; q0 += 4) {
+      double v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        v[q] = __ldg(W + (int64_t)(32 * w + min(q0 + q, i1 - 1)) * M);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q0 + q < i1) {
+          const uint32_t flip = (bits >> (q0 + q)) & 1u ? 0u : 0x80000000u;
+          th += __hiloint2double(__double2hiint(v[q]) ^ (int)flip, __double2loint(v[q]));
+        }
+    }
+  }
+  return th;
+}
+
+// The plain kernel's decision in FP64, theta formed from scratch for the spins in the
+// words xb (word l in lane l).  MANY hidden units per lane: s as a sum of |t| - |theta|
+// and one logarithm of a quotient of products per lane, half the FP64 operations of a
+// log_cosh per hidden unit.  The launch ends with the chain that meets the most of these:
+// 1,024 chains, N = 64, M = 128: 314 -> 245 us (one load at a time and log_cosh before;
+// 275 with log_cosh); N = 36, M = 72: 246 -> 228 us; one unit per lane (N = M = 16): 234
+// with log_cosh, 253 without.
+template <bool MANY>
 __device__ __noinline__ bool exact_accept_f64(const double *__restrict__ params, int N, int M,
                                               uint32_t xb, int su, int sv, int du, int hop,
                                               int hop_new, uint32_t ry, uint32_t rz) {
   const int lane = threadIdx.x & 31;
   const double *W = params + M, *a = params + M + (int64_t)N * M;
-  double s = 0.0;
+  double s = 0.0, p_new = 1.0, p_old = 1.0;
   for (int j0 = 0; j0 < M; j0 += 32) {
-    const int j = j0 + lane;
-    const bool in = j < M;
-    const double *Wj = W + (in ? j : 0);
-    double th = in ? params[j] : 0.0;
-    for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-      const int i1 = min(32, N - 32 * w);
-      for (int q = 0; q < i1; ++q) {
-        const double v = Wj[(int64_t)(32 * w + q) * M];
-        th += (bits >> q) & 1u ? v : -v;
+    const int j = j0 + lane < M ? j0 + lane : -1;
+    const double th = theta_f64(params, N, M, xb, j);
+    if (j >= 0) {
+      double t = th + (double)du * W[(int64_t)su * M + j];
+      if (sv >= 0) t -= (double)du * W[(int64_t)sv * M + j];
+      if (MANY) {
+        s += fabs(t) - fabs(th);
+        p_new = fma(p_new, exp(-2.0 * fabs(t)), p_new);  // at most 2^(M / 32)
+        p_old = fma(p_old, exp(-2.0 * fabs(th)), p_old);
+      } else {
+        s += log_cosh(t) - log_cosh(th);
       }
     }
-    if (in) {
-      double t = th + (double)du * Wj[(int64_t)su * M];
-      if (sv >= 0) t -= (double)du * Wj[(int64_t)sv * M];
-      s += log_cosh(t) - log_cosh(th);
-    }
   }
+  if (MANY) s += log(p_new / p_old);
   s = warp_sum(s);
   s += (double)du * a[su];
   double corr = 0.0;
@@ -59,22 +87,12 @@ __device__ __noinline__ bool exact_accept_f64(const double *__restrict__ params,
 __device__ __noinline__ double final_logpsi_f64(const double *__restrict__ params, int N, int M,
                                                 uint32_t xb) {
   const int lane = threadIdx.x & 31;
-  const double *W = params + M, *a = params + M + (int64_t)N * M;
+  const double *a = params + M + (int64_t)N * M;
   double part = 0.0;
   for (int j0 = 0; j0 < M; j0 += 32) {
-    const int j = j0 + lane;
-    const bool in = j < M;
-    const double *Wj = W + (in ? j : 0);
-    double th = in ? params[j] : 0.0;
-    for (int w = 0; 32 * w < N; ++w) {
-      const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);
-      const int i1 = min(32, N - 32 * w);
-      for (int q = 0; q < i1; ++q) {
-        const double v = Wj[(int64_t)(32 * w + q) * M];
-        th += (bits >> q) & 1u ? v : -v;
-      }
-    }
-    if (in) part += log_cosh(th);
+    const int j = j0 + lane < M ? j0 + lane : -1;
+    const double th = theta_f64(params, N, M, xb, j);
+    if (j >= 0) part += log_cosh(th);
   }
   for (int w = 0; 32 * w < N; ++w) {
     const uint32_t bits = __shfl_sync(0xffffffffu, xb, w);

@@ -32,9 +32,9 @@
 //
 // Measured (GB300, MCState.sample, before -> now; before = one log_cosh per hidden
 // unit and proposal): FP64 Local, N = 64, M = 128, 1,024 chains x 9 sweeps 14.1 ->
-// 0.67 ms; FP64 Exchange, N = 36, M = 72, 1,024 chains 7.77 -> 0.52 ms; FP32
-// Exchange, 10 x 10 J1-J2, M = 400, 4,096 chains 3.45 -> 1.22 ms (about 880 warp
-// instructions per proposal before).
+// 0.28 ms; FP64 Exchange, N = 36, M = 72, 1,024 chains 7.77 -> 0.23 ms; FP32
+// Exchange, 10 x 10 J1-J2, M = 400, 4,096 chains 3.45 -> 1.10 ms (about 880 warp
+// instructions per proposal before, 312 now).
 #include <algorithm>
 
 #include "filter_common.cuh"
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
       if (!(fabsf(margin) > eps) || __any_sync(0xffffffffu, far)) {
         // too close to call: the plain kernel's own evaluation
         if constexpr (F64) {
-          accept = exact_accept_f64(static_cast<const double *>(A.params), N, M, ch.xb, su,
+          accept = exact_accept_f64<(R > 1)>(static_cast<const double *>(A.params), N, M, ch.xb, su,
                                     sv, du, ch.hop, pr.hop_new,
                                     __shfl_sync(0xffffffffu, rnd.y, p & 31),
                                     __shfl_sync(0xffffffffu, rnd.z, p & 31));

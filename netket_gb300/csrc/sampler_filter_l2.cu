@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(32 * l2_warps<T, Q>(), 1)
         bool accept = margin < 0.0f;
         if (!(fabsf(margin) > eps) || __any_sync(0xffffffffu, far)) {
           if constexpr (F64) {
-            accept = exact_accept_f64(static_cast<const double *>(A.params), N, M, ch.xb, su, sv,
+            accept = exact_accept_f64<true>(static_cast<const double *>(A.params), N, M, ch.xb, su, sv,
                                       du, ch.hop, pr.hop_new,
                                       __shfl_sync(0xffffffffu, rnd.y, p & 31),
                                       __shfl_sync(0xffffffffu, rnd.z, p & 31));
