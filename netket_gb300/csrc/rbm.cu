@@ -215,7 +215,8 @@ __device__ inline T warp_log_ratio(const RbmParams<T> &P, const T *th, const T *
 
 // Local energy of one sample for the Ising Hamiltonian, by the whole CTA.
 // xs must hold the configuration (visible to all threads); returns E_loc on
-// every thread.
+// every thread.  FP32: the sums of eloc_f32_kernel in its order, so that a batched
+// instance's energies are those of the instance alone, bit for bit.
 template <typename T>
 __device__ double eloc_ising_sample(const RbmParams<T> &P, const int8_t *xs,
                                     const int32_t *__restrict__ edges, int n_edges, double h,
@@ -234,8 +235,17 @@ __device__ double eloc_ising_sample(const RbmParams<T> &P, const int8_t *xs,
       int site = k;
       T d = (T)(-2 * xs[k]);
       T lr = warp_log_ratio(P, th, lc, &site, &d, 1);
-      if (lane == 0) acc += -h * exp_ratio(lr);
+      // FP32: four partial sums per warp, as eloc_f32_kernel's four elements at a time
+      const int owner = sizeof(T) == 4 ? 8 * ((k / nw) & 3) : 0;
+      if (lane == owner) acc += -h * exp_ratio(lr);
     }
+  }
+  if (sizeof(T) == 4 && nw == 4) {
+    acc = warp_sum(acc);
+    __syncthreads();
+    if (lane == 0) redd[warp] = acc;
+    __syncthreads();
+    return ((redd[0] + redd[1]) + (redd[2] + redd[3])) + J * (double)tot;
   }
   if (threadIdx.x == 0) acc += J * (double)tot;
   return block_sum(acc, redd);
