@@ -87,6 +87,14 @@ __device__ __forceinline__ void fill_table(T *tab, T w0, T w1, T w2, T w3) {
   tab[15 * 32] = -ps;
 }
 
+// a + b, its rounding error added to low (infinities and NaN reach the sum alone)
+__device__ __forceinline__ double two_sum(double a, double b, double &low) {
+  const double s = a + b, v = s - a;
+  const double e = (a - (s - v)) + (b - v);
+  if (isfinite(s)) low += e;
+  return s;
+}
+
 enum RowsOut { ROWS_LOGPSI = 0, ROWS_DOT = 1, ROWS_THETA = 2 };
 
 // A cluster takes SR_WARPS * SPW samples; its CTAs share the tiles of 32 hidden units
@@ -103,7 +111,7 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
     double *__restrict__ theta_out, double *__restrict__ tanh_out, u64 *__restrict__ q_out) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint32_t largest[SR_WARPS][32];
-  __shared__ double sum[SR_WARPS * SPW];
+  __shared__ double sum[2 * SR_WARPS * SPW];  // sums, their low parts
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
   const int G = (N + 3) >> 2, G4 = (G + 3) & ~3, bits = sum_bits(N);
@@ -253,27 +261,51 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
     }
   }
   if constexpr (OUT != ROWS_THETA) {
+    // log psi is a sum of hundreds that its callers subtract from another: its last
+    // additions are kept with their errors
+    double low[SPW];
 #pragma unroll
-    for (int s = 0; s < SPW; ++s)  // at most 2^(M / 32) per lane; log 2 taken out exactly
-      if (OUT == ROWS_LOGPSI) acc[s] += log(ldexp(prod[s], -units));
+    for (int s = 0; s < SPW; ++s) {
+      low[s] = 0.0;  // at most 2^(M / 32) per lane; log 2 taken out exactly
+      if (OUT == ROWS_LOGPSI) acc[s] = two_sum(acc[s], log(ldexp(prod[s], -units)), low[s]);
+    }
     if (rank == 0)
       for (int i = lane; i < N; i += 32) {
         const double ai = __ldg(a + i);
 #pragma unroll
         for (int s = 0; s < SPW; ++s)
-          if (sw + s < n) acc[s] += x[(sw + s) * N + i] < 0 ? -ai : ai;
+          if (sw + s < n) {
+            const double v = x[(sw + s) * N + i] < 0 ? -ai : ai;
+            acc[s] = OUT == ROWS_LOGPSI ? two_sum(acc[s], v, low[s]) : acc[s] + v;
+          }
       }
 #pragma unroll
     for (int s = 0; s < SPW; ++s) {
-      const double v = warp_sum(acc[s]);
-      if (lane == 0) sum[warp * SPW + s] = v;
+      if (OUT == ROWS_LOGPSI) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const double v = __shfl_xor_sync(0xffffffffu, acc[s], o);
+          low[s] += __shfl_xor_sync(0xffffffffu, low[s], o);
+          acc[s] = two_sum(acc[s], v, low[s]);
+        }
+      } else {
+        acc[s] = warp_sum(acc[s]);
+      }
+      if (lane == 0) {
+        sum[warp * SPW + s] = acc[s];
+        sum[SR_WARPS * SPW + warp * SPW + s] = low[s];
+      }
     }
     if (ranks > 1) cluster.sync();
     else __syncthreads();
     if (rank == 0 && tid < SR_WARPS * SPW && s0 + tid < n) {
-      double v = sum[tid];
-      for (int r = 1; r < ranks; ++r) v += cluster.map_shared_rank(sum, r)[tid];
-      out[s0 + tid] = v;
+      double v = sum[tid], l = sum[SR_WARPS * SPW + tid];
+      for (int r = 1; r < ranks; ++r) {
+        const double *other = cluster.map_shared_rank(sum, r);
+        v = two_sum(v, other[tid], l);
+        l += other[SR_WARPS * SPW + tid];
+      }
+      out[s0 + tid] = v + l;
     }
     if (ranks > 1) cluster.sync();  // the others' sums stay until they are read
   }
