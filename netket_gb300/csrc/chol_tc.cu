@@ -1129,7 +1129,11 @@ int chol_tc_factor(cudaStream_t st, float *A, int64_t n, void *ws, int32_t *stat
   // and two refinements 11.87 -> 11.30 ms; 11.75 with none left, 11.36 with four, 11.63
   // with sixteen; n = 24,000: 27.7 -> 26.35).  Before the first trailing update the
   // whole chip is the chain's, and a reserve there changes nothing.
-  const int chain2_grid = std::max(8, num_sms_dev() - side_grid - 2);
+  // From CHOL_BIG_N on, with 24 SMs reserved, 22 are too few for the updates once the side
+  // stream is done: the whole grid (32,768 / 40,960 / 49,152: 54.5 / 95 / 150 ms; limited
+  // 55.3 / 95 / 194).
+  const int chain2_grid =
+      n >= CHOL_BIG_N ? 0 : std::max(8, num_sms_dev() - side_grid - 2);
   VMCK_CUDA(cudaFuncSetAttribute(chol_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)CHOL_LEAF_SMEM));
   // the leaf writes X and Y on and above, or below, their diagonals
