@@ -255,13 +255,14 @@ __device__ __forceinline__ int fold_length(int s8, int s4, int s2, int &s) {
 }
 
 // ------------------------------------------------------------ Ising
-// One CTA takes S samples: their q in shared memory, then each warp takes pairs of sites: one read of the two sites' table rows serves all
+// One CTA takes S samples (gridDim.y CTAs share their sites): their q in shared memory,
+// then each warp takes pairs of sites: one read of the two sites' table rows serves all
 // samples, one read of a sample's q both sites, and four products are reduced together
 // (warp_prod4).  Lane group e accumulates sample e's (and e + 4's) sum.
-// N = 256, M = 256, n = 2,048: 0.35 ms with the tables and theta (products in FP64
+// N = 256, M = 256, n = 2,048: 0.34 ms with the tables and theta (products in FP64
 // 1.14 ms; one log_cosh per hidden unit and flip, eloc_ising_kernel<double>, 20.1 ms).
 // The issue of the integer products bounds it: 42 % of the slots at 16 warps per SM,
-// whatever the split of samples and sites (four, eight; one, two: 280 to 310 us).
+// whatever a warp's samples and sites (four, eight; one, two).
 template <int S>
 constexpr int ising_threads() {
   return S == 8 ? 256 : 128;
@@ -324,7 +325,7 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
         for (int s = warp; s < S; s += WARPS) norm[s][lane] = lane_norm(rho + s * M, M);
         __syncthreads();
       }
-      for (int k0 = 2 * warp; k0 < N; k0 += 2 * WARPS) {
+      for (int k0 = 2 * (WARPS * (int)blockIdx.y + warp); k0 < N; k0 += 2 * WARPS * gridDim.y) {
         // site k0 + 1 = N stands for the row of ones
         int bits[2];  // bit s: sample s's spin of site k0 + t is down
         int fold = finite ? 8 : 0, S8 = 0, S4 = 0, S2 = 0, range = 0;
@@ -351,28 +352,31 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
             for (int s = 0; s < 4 * W4; ++s) g[t][s] = lane_one(range);
           const u64 *up = tab.uup + (int64_t)k0 * M, *down = tab.udown + (int64_t)k0 * M;
 #pragma unroll 1
-          for (int j = lane; j < M; j += 32) {
-            if (count == fold) {
+          for (int js = 0; js < M; js += 32 * fold) {
+            if (js > 0) {
 #pragma unroll
               for (int t = 0; t < 2; ++t)
 #pragma unroll
                 for (int s = 0; s < S; ++s) g[t][s] = lane_renew(g[t][s], count, range);
-              count = 0;
             }
-            ++count;
-            u64 u[2][2];
-#pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              u[t][0] = __ldg(down + (int64_t)t * M + j);
-              u[t][1] = __ldg(up + (int64_t)t * M + j);
-            }
-#pragma unroll
-            for (int s = 0; s < S; ++s) {
-              const u64 q = qs[s * M + j], p = (offset - q) >> 4;
+            const int je = min(M, js + 32 * fold);
+            count = (je - js - lane + 31) >> 5;
+#pragma unroll 1
+            for (int j = js + lane; j < je; j += 32) {
+              u64 u[2][2];
 #pragma unroll
               for (int t = 0; t < 2; ++t) {
-                const u64 ut = (bits[t] >> s) & 1 ? u[t][1] : u[t][0];
-                g[t][s].f = times_factor<60>(g[t][s].f, factor<60>(q, ut, p));
+                u[t][0] = __ldg(down + (int64_t)t * M + j);
+                u[t][1] = __ldg(up + (int64_t)t * M + j);
+              }
+#pragma unroll
+              for (int s = 0; s < S; ++s) {
+                const u64 q = qs[s * M + j], p = (offset - q) >> 4;
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                  const u64 ut = (bits[t] >> s) & 1 ? u[t][1] : u[t][0];
+                  g[t][s].f = times_factor<60>(g[t][s].f, factor<60>(q, ut, p));
+                }
               }
             }
           }
@@ -434,7 +438,11 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
       double s = 0.0;
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) s += red[w][tid];
-      eloc[b0 + tid] = (h != 0.0 ? -h * s : 0.0) + J * (double)diag[tid];
+      const double e = h != 0.0 ? -h * s : 0.0;
+      if (gridDim.y == 1)
+        eloc[b0 + tid] = e + J * (double)diag[tid];
+      else  // two addends and zero: their order does not matter
+        atomicAdd(eloc + b0 + tid, blockIdx.y == 0 ? e + J * (double)diag[tid] : e);
     }
     __syncthreads();
   }
@@ -445,7 +453,7 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
 // enumerated in shared memory (local_conn_enumerate), then each warp takes groups
 // of four elements: NS table rows each (a site that the element leaves alone
 // reads the row of ones), four products reduced together.  10 x 10 Heisenberg, M = 200,
-// n = 4,096 (about 100 elements a sample): 0.40 ms with the tables and theta (products in
+// n = 4,096 (about 100 elements a sample): 0.38 ms with the tables and theta (products in
 // FP64 1.02 ms; eloc_local_kernel<double> 14.4 ms).
 template <int NS>
 __global__ void __launch_bounds__(EF_THREADS) eloc_local_f64_kernel(
@@ -529,32 +537,35 @@ __global__ void __launch_bounds__(EF_THREADS) eloc_local_f64_kernel(
         constexpr int B = NS == 1 ? 60 : 56;  // units of an element's u
         const u64 offset = p_offset<B>(lane);
         LaneProduct g[4];
-        int count = 0;
+        int count = 0;  // factors since g was scaled
 #pragma unroll
         for (int e = 0; e < 4; ++e) g[e] = lane_one(range);
 #pragma unroll 1
-        for (int j = lane; j < M; j += 32) {
-          if (count == fold) {
+        for (int js = 0; js < M; js += 32 * fold) {
+          if (js > 0) {
 #pragma unroll
             for (int e = 0; e < 4; ++e) g[e] = lane_renew(g[e], count, range);
-            count = 0;
           }
-          ++count;
-          u64 u[4][NS];
+          const int je = min(M, js + 32 * fold);
+          count = (je - js - lane + 31) >> 5;
+#pragma unroll 2
+          for (int j = js + lane; j < je; j += 32) {
+            u64 u[4][NS];
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
+            for (int e = 0; e < 4; ++e)
 #pragma unroll
-            for (int q = 0; q < NS; ++q) u[e][q] = __ldg(tab.uup + row[e][q] + j);
-          const u64 q = qs[j], p = (offset - q) >> (64 - B);
+              for (int q = 0; q < NS; ++q) u[e][q] = __ldg(tab.uup + row[e][q] + j);
+            const u64 q = qs[j], p = (offset - q) >> (64 - B);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            u64 ue = u[e][0];
-            if (NS == 2) {
-              uint32_t below;
-              ue = mul_high(ue, u[e][NS - 1], below);
-              ue += below >> 31;
+            for (int e = 0; e < 4; ++e) {
+              u64 ue = u[e][0];
+              if (NS == 2) {
+                uint32_t below;
+                ue = mul_high(ue, u[e][NS - 1], below);
+                ue += below >> 31;
+              }
+              g[e].f = times_factor<B>(g[e].f, factor<B>(q, ue, p));
             }
-            g[e].f = times_factor<B>(g[e].f, factor<B>(q, ue, p));
           }
         }
         UFloat quad[4];
@@ -640,13 +651,14 @@ static size_t ising_smem(int S, int N, int M) {
 template <int S>
 static int launch_ising(cudaStream_t st, const double *params, int N, int M, const int8_t *x,
                         int64_t n, const int32_t *edges, int n_edges, double h, double J,
-                        const FlipTables &tab, double *eloc) {
+                        const FlipTables &tab, double *eloc, int split) {
   const size_t smem = ising_smem(S, N, M);
   if (smem > 40 * 1024)
     VMCK_CUDA(cudaFuncSetAttribute(eloc_ising_f64_kernel<S>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t grid = std::min<int64_t>((n + S - 1) / S, (int64_t)sm_count() * 32);
-  eloc_ising_f64_kernel<S><<<(unsigned)grid, ising_threads<S>(), smem, st>>>(
+  if (split == 2) VMCK_CUDA(cudaMemsetAsync(eloc, 0, (size_t)n * 8, st));
+  eloc_ising_f64_kernel<S><<<dim3((unsigned)grid, split), ising_threads<S>(), smem, st>>>(
       params, N, M, x, n, edges, n_edges, h, J, tab, eloc);
   return check_launch("rbm_eloc_ising_f64");
 }
@@ -694,13 +706,18 @@ extern "C" int vmck_rbm_eloc_ising_f64(vmck_stream s, const double *params, int3
   for (int64_t c = 0; c < n; c += chunk, x += chunk * N, eloc += chunk) {
     const int64_t m = std::min(chunk, n - c);
     if (h != 0.0 && (rc = theta_q_f64(st, params, N, M, x, m, tab.theta, tab.q))) return rc;
-    // eight samples share a pass over the tables; four while eight leave SMs empty
-    if (m > 8 * (int64_t)sm_count() && ising_smem(8, N, M) <= EF_SMEM_MAX / 2)
-      rc = launch_ising<8>(st, params, N, M, x, m, edges, n_edges, h, J, tab, eloc);
+    // Eight samples share a read of the tables, four while there are few.  Two CTAs share a
+    // sample group's sites where each warp still has two pairs of them: the last round of
+    // CTAs is shorter.  N = M = 256, n = 1,500 / 2,048 / 3,000 / 4,096 / 16,384: 350 / 352 /
+    // 509 / 626 / 2,038 us with eight and no split, 305 / 340 / 437 / 565 / 1,998 so; N =
+    // 32, M = 64: 40 us without the split, 45 with it.
+    const int split = h != 0.0 && N >= 64 ? 2 : 1;
+    if (m > 16 * (int64_t)sm_count() && ising_smem(8, N, M) <= EF_SMEM_MAX / 2)
+      rc = launch_ising<8>(st, params, N, M, x, m, edges, n_edges, h, J, tab, eloc, split);
     else if (ising_smem(4, N, M) <= EF_SMEM_MAX)
-      rc = launch_ising<4>(st, params, N, M, x, m, edges, n_edges, h, J, tab, eloc);
+      rc = launch_ising<4>(st, params, N, M, x, m, edges, n_edges, h, J, tab, eloc, split);
     else
-      rc = launch_ising<2>(st, params, N, M, x, m, edges, n_edges, h, J, tab, eloc);
+      rc = launch_ising<2>(st, params, N, M, x, m, edges, n_edges, h, J, tab, eloc, 1);
     if (rc) return rc;
   }
   return VMCK_OK;

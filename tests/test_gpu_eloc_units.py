@@ -1,8 +1,8 @@
 """The fixed-point form of the FP64 local energies (eloc_f64.cu) against the oracle where
 it changes course: hidden widths around the 32 lanes and the eight factors of a lane
 between two scalings, weights that ask for four or two factors or for the FP64 form in
-some rows, theta at the ends of q, eight, four and two samples per CTA, more samples than
-a chunk.
+some rows, theta at the ends of q, eight, four and two samples per CTA, sites shared by
+two CTAs (from 64 sites on), more samples than a chunk.
 
 Tolerance 1e-11 relative: M <= 4,000 factors within 2^-53 are 5e-13, the oracle's
 log_cosh sums M |theta| 2^-53 <= 600 x 40 x 1.1e-16 = 3e-12."""
@@ -35,7 +35,7 @@ def _check(H, get_conn, flat, x, N, M):
     (6, 31, 40, 0.05, 0.0), (9, 33, 1500, 0.1, 0.0), (5, 257, 30, 0.05, 0.0),
     (7, 520, 13, 0.02, 0.0), (8, 300, 20, 0.15, 0.0), (11, 64, 21, 0.6, 0.0),
     (4, 2000, 9, 0.01, 0.0), (3, 4000, 5, 0.01, 0.0), (4, 8, 16390, 0.1, 0.0),
-    (6, 40, 1300, 0.1, 30.0)])
+    (6, 40, 1300, 0.1, 30.0), (64, 40, 50, 0.05, 0.0), (65, 33, 2500, 0.03, 0.0)])
 def test_ising(N, M, n, std, bias):
     import netket_gb300 as nk
     hi, g = nk.hilbert.Spin(0.5, N), nk.graph.Chain(N, pbc=N > 2)
