@@ -222,6 +222,17 @@ __device__ __forceinline__ T block_sum(T v, T *red) {
   return t;
 }
 
+// SMs of the device, asked for once (a launch's grid alone depends on it)
+inline int sm_count() {
+  static const int sms = [] {
+    int dev = 0, n = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n;
+  }();
+  return sms;
+}
+
 template <typename T>
 struct Real;
 template <>

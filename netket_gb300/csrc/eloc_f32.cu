@@ -292,13 +292,12 @@ template <bool ISING, bool WSM, bool VEC>
 static int launch_e3(cudaStream_t st, const float *params, int N, int M, const int8_t *x,
                      int64_t n, const vmck_local_op &op, const IsingArgs &ising, int cap,
                      int groups, double *eloc) {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = sm_count();
   const E3Smem s = e3_smem(WSM, N, M, cap);
   const size_t smem = s.group + groups * s.per_group;
-  VMCK_CUDA(cudaFuncSetAttribute(eloc_f32_kernel<ISING, WSM, VEC>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 40 * 1024)
+    VMCK_CUDA(cudaFuncSetAttribute(eloc_f32_kernel<ISING, WSM, VEC>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t grid = WSM ? std::min<int64_t>((n + groups - 1) / groups, sms)
                            : std::min<int64_t>(n, (int64_t)sms * 32);
   eloc_f32_kernel<ISING, WSM, VEC><<<(unsigned)grid, E3_GROUP * groups, smem, st>>>(
@@ -321,9 +320,14 @@ static int e3_any(cudaStream_t st, const float *params, int N, int M, const int8
   const E3Smem s = e3_smem(true, N, M, cap);
   int groups = s.group < E3_SMEM_MAX ? (int)((E3_SMEM_MAX - s.group) / s.per_group) : 0;
   groups = std::min(groups, E3_MAX_GROUPS);
-  // weights in shared memory from four groups up (16 warps) and where every SM gets
-  // a few samples to pay for the copy
-  if (groups >= 4 && n >= 1024)
+  // Weights in shared memory where at least four groups (16 warps) fit beside them and the
+  // connected elements are many enough to pay for the copy and for the warps that do not
+  // fit: about a million single-site ones, 0.75 million of samples with 128 and more (half
+  // of the terms).  L2 / shared memory, us: Ising N = 100, M = 400: n = 3,000 136 / 147,
+  // 16,384 672 / 571; J1-J2 8 x 8, M = 256: 3,000 114 / 120, 6,000 205 / 196; 10 x 10, M = 400:
+  // 16,384 1,360 / 1,172; Heisenberg 10 x 10 (200 terms), M = 500: 16,384 1,044 / 1,100.
+  const bool many = ISING ? n * N >= 1000000 : op.n_terms >= 256 && n * op.n_terms >= 1500000;
+  if (groups >= 4 && many)
     return launch_e3<ISING, true, true>(st, params, N, M, x, n, op, ising, cap, groups, eloc);
   const bool vec = M % 4 == 0 && reinterpret_cast<uintptr_t>(params) % 16 == 0;
   return vec ? launch_e3<ISING, false, true>(st, params, N, M, x, n, op, ising, cap, 1, eloc)
@@ -332,8 +336,12 @@ static int e3_any(cudaStream_t st, const float *params, int N, int M, const int8
 
 // Terms of at most two sites, sites in 14 bits, and the lists in shared memory; what
 // the general kernel's vectors do not fit stays refused by it.
-bool eloc_f32_takes(int N, int M, const vmck_local_op *op) {
+bool eloc_f32_takes(int N, int M, int64_t n, const vmck_local_op *op) {
   if (N >= (1 << 14)) return false;
+  // a handful of samples with wide layers wait for W from L2 either way; the general kernel
+  // has more of its rows in flight (12 x 12 J1-J2, M = 1,152: n = 600 336 us here, 333 there;
+  // n = 5,000 1,553 here, 1,941 there)
+  if (M >= 1024 && n <= 4 * (int64_t)sm_count()) return false;
   const size_t general =
       2 * 4 * (size_t)M + (op ? local_conn_shared_bytes(*op) + 16 : align16((size_t)N));
   if (general > 200 * 1024) return false;

@@ -36,6 +36,7 @@ namespace vmck {
 
 constexpr int EF_THREADS = 128, EF_WARPS = EF_THREADS / 32;  // LocalOperator
 constexpr int EF_S_MAX = 8;
+constexpr int EF_DIRECT = 12;
 constexpr int64_t EF_CHUNK = 16384;  // samples whose theta and q are kept at once
 
 // Tables of the call: up[i, j] = exp(-4 W_ij) and down[i, j] = exp(4 W_ij), the
@@ -631,13 +632,6 @@ __global__ void __launch_bounds__(EF_THREADS) eloc_local_f64_kernel(
   }
 }
 
-static int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 static int launch_flip_tables(cudaStream_t st, const double *params, int N, int M, double *ws) {
   flip_tables_kernel<<<N + 1, 256, 0, st>>>(params, N, M, ws);
   return check_launch("flip tables");
@@ -694,9 +688,12 @@ extern "C" int vmck_rbm_eloc_ising_f64(vmck_stream s, const double *params, int3
   VMCK_REQUIRE(workspace_len >= flip_table_len(N, M, n), "rbm_eloc_ising_f64 workspace too small");
   if (n == 0) return VMCK_OK;
   cudaStream_t st = as_stream(s);
-  // (two samples' vectors do not fit, or the sites' sign indices: one log_cosh per hidden
-  // unit)
-  if (ising_smem(2, N, M) > EF_SMEM_MAX || !signed_rows_fit(N))
+  // One log_cosh per hidden unit and flip where that is a single launch of a few us (at most
+  // EF_DIRECT warp rounds of flips per SM: n = 16, N = M = 8: 17 us a call, 28 by the three
+  // launches below; N = M = 16: 44 and 46; N = M = 24: 52 and 48), and where two samples'
+  // vectors or the sites' sign indices do not fit.
+  const int64_t rounds = (n + sm_count() - 1) / sm_count() * N * ((M + 31) / 32);
+  if (rounds <= EF_DIRECT || ising_smem(2, N, M) > EF_SMEM_MAX || !signed_rows_fit(N))
     return vmck_rbm_eloc_ising(s, VMCK_F64, params, N, M, x, n, edges, n_edges, h, J, eloc,
                                nullptr);
   int rc;

@@ -12,13 +12,6 @@ namespace vmck {
 
 constexpr int PS_THREADS = 256;
 
-static int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 __global__ void __launch_bounds__(PS_THREADS)
     get_conn_pauli_kernel(vmck_pauli_strings op, const int8_t *__restrict__ x, int64_t n,
                           int8_t *xp, double *mels, int32_t *n_conn) {

@@ -715,7 +715,7 @@ extern "C" int vmck_rbm_eloc_ising(vmck_stream s, int32_t dtype, const void *par
   if (dtype == VMCK_F64)
     return launch_eloc_ising<double>(as_stream(s), params, N, M, x, n, edges, n_edges, h, J,
                                      eloc, logpsi_out);
-  if (dtype == VMCK_F32 && !logpsi_out && eloc_f32_takes(N, M, nullptr))
+  if (dtype == VMCK_F32 && !logpsi_out && eloc_f32_takes(N, M, n, nullptr))
     return eloc_f32_ising(as_stream(s), static_cast<const float *>(params), N, M, x, n, edges,
                           n_edges, h, J, eloc);
   if (dtype == VMCK_F32)
@@ -735,7 +735,7 @@ extern "C" int vmck_rbm_eloc_local(vmck_stream s, int32_t dtype, const void *par
   if (n == 0) return VMCK_OK;
   if (dtype == VMCK_F64)
     return launch_eloc_local<double>(as_stream(s), params, N, M, x, n, *op, eloc, logpsi_out);
-  if (dtype == VMCK_F32 && !logpsi_out && eloc_f32_takes(N, M, op))
+  if (dtype == VMCK_F32 && !logpsi_out && eloc_f32_takes(N, M, n, op))
     return eloc_f32_local(as_stream(s), static_cast<const float *>(params), N, M, x, n, *op, eloc);
   if (dtype == VMCK_F32)
     return launch_eloc_local<float>(as_stream(s), params, N, M, x, n, *op, eloc, logpsi_out);

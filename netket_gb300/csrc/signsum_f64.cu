@@ -311,13 +311,6 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
   }
 }
 
-int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
-
 template <RowsOut OUT, int SPW>
 int launch_rows_as(cudaStream_t st, int ranks, const double *params, const int8_t *x, int N, int M,
                    int64_t n, const double *t, double *out, double *theta, double *tanh_out,
@@ -327,8 +320,9 @@ int launch_rows_as(cudaStream_t st, int ranks, const double *params, const int8_
   const int blocks = G <= SR_BLOCK ? 1 : (G + 23) / 24;
   const int block = blocks == 1 ? G : ((G + blocks - 1) / blocks + 3) & ~3;
   const size_t smem = (size_t)block * SS_TAB * 8 + (size_t)SR_WARPS * SPW * G4;
-  VMCK_CUDA(cudaFuncSetAttribute(signed_rows_kernel<OUT, SPW>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 40 * 1024)
+    VMCK_CUDA(cudaFuncSetAttribute(signed_rows_kernel<OUT, SPW>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t grid = (n + SR_WARPS * SPW - 1) / (SR_WARPS * SPW) * ranks;
   VMCK_REQUIRE(grid < (1ll << 31), "too many rows");
   cudaLaunchAttribute attr[1];
@@ -341,7 +335,7 @@ int launch_rows_as(cudaStream_t st, int ranks, const double *params, const int8_
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = ranks > 1;
   VMCK_CUDA(cudaLaunchKernelEx(&cfg, signed_rows_kernel<OUT, SPW>, params, x, N, M, n, block, t,
                                out, theta, tanh_out, q));
   return check_launch("rows of signed sums");

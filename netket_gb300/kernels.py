@@ -65,7 +65,9 @@ def local_energies_fused(op, params_c, x, N, M):
         nat.check(nat.lib().vmck_rbm_eloc_pauli(nat.stream(), dt, nat.ptr(params_c), N, M,
                                                 nat.ptr(x), n, ctypes.byref(st), nat.ptr(e), None))
         return e
-    if params_c.dtype == torch.float64 and isinstance(op, (Ising, LocalOperator)):
+    # (a few single flips: one launch of the direct kernel, without a workspace, is quicker)
+    few = isinstance(op, Ising) and n <= 128 and N * -(-M // 32) <= 12
+    if params_c.dtype == torch.float64 and isinstance(op, (Ising, LocalOperator)) and not few:
         ws = torch.empty(nat.lib().vmck_rbm_eloc_f64_workspace_size(N, M, n),
                          dtype=torch.float64, device=x.device)
         if isinstance(op, Ising):

@@ -45,7 +45,8 @@ def _check(op, N, M, n, std=0.2, total_sz=None):
 
 @pytest.mark.parametrize("N,M,n", [(2, 1, 1), (5, 31, 3), (9, 32, 1030), (16, 33, 1024),
                                    (33, 100, 1500), (100, 400, 1100), (64, 259, 40),
-                                   (100, 512, 1030), (256, 256, 30)])
+                                   (100, 512, 1030), (256, 256, 30), (128, 40, 8000),
+                                   (33, 100, 31000)])
 def test_ising(N, M, n):
     import netket_gb300 as nk
     hi = nk.hilbert.Spin(0.5, N)
@@ -54,7 +55,8 @@ def test_ising(N, M, n):
 
 @pytest.mark.parametrize("L,M,n,std", [(4, 7, 5, 0.2), (4, 32, 1027, 0.01), (6, 66, 1024, 0.3),
                                        (6, 144, 100, 3.0), (10, 400, 1100, 0.05),
-                                       (10, 402, 33, 0.05), (10, 800, 20, 0.05)])
+                                       (10, 402, 33, 0.05), (10, 800, 20, 0.05),
+                                       (10, 66, 3751, 0.3), (10, 400, 3800, 0.05)])
 def test_heisenberg(L, M, n, std):
     import netket_gb300 as nk
     hi = nk.hilbert.Spin(0.5, L * L, total_sz=0)
