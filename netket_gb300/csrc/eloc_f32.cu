@@ -11,8 +11,8 @@
 // Here eight lanes take one element, lane l holding the partial sums 4 l .. 4 l + 3:
 // operands come in 16-byte loads and one butterfly serves the four elements of a
 // warp.  Weights that fit are kept in shared memory (one CTA per SM, several
-// groups of four warps, each with its own sample and barrier); the others are read
-// through L1.  Each warp lists the connected elements of its share of the terms
+// groups of four warps, each with its own sample and barrier) where the elements are many
+// enough (e3_any); the others are read through L1.  Each warp lists the connected elements of its share of the terms
 // by ballots, with nothing shared between warps before the sample's sum.
 //
 // What bounds it: FP32 issue (27 instructions per 32 hidden units of an element).
