@@ -52,6 +52,7 @@ constexpr int SR_HELD = 4;       // groups of a warp held in registers
 constexpr int SR_BLOCK = 26;     // groups per table block: two CTAs' tables in an SM
 constexpr int64_t SR_INDEX_MAX = 32 * 1024;  // bytes of sign indices per CTA
 constexpr int SR_SITES_MAX = 16384;
+constexpr int SR_FOLD = 512;  // hidden units of a lane between two logarithms of log psi
 
 // acc + the table's entry number `byte` (a byte of four, moved to bits 8 to 11: the
 // entries are 256 bytes apart)
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
   const uint8_t *mine = index + (size_t)warp * SPW * G4;
   const int64_t sw = s0 + warp * SPW;  // this warp's first sample
   double acc[SPW], prod[SPW];
-  int units = 0;  // this lane's hidden units
+  int units = 0;  // this lane's hidden units in prod
 #pragma unroll
   for (int s = 0; s < SPW; ++s) {
     acc[s] = 0.0;
@@ -259,6 +260,16 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
       }
       if (theta_out) theta_out[row * M + j] = th[s];
     }
+    // 1 + e^(-2|theta|) is up to 2: without this, prod leaves the double range at 1,024 units
+    // of a lane (M = 65,536).  A lane comes here from M = 32,705 on.
+    if (OUT == ROWS_LOGPSI && units == SR_FOLD) {
+#pragma unroll
+      for (int s = 0; s < SPW; ++s) {
+        acc[s] += log(ldexp(prod[s], -SR_FOLD));
+        prod[s] = 1.0;
+      }
+      units = 0;
+    }
   }
   if constexpr (OUT != ROWS_THETA) {
     // log psi is a sum of hundreds that its callers subtract from another: its last
@@ -266,7 +277,7 @@ __global__ void __launch_bounds__(SR_THREADS, 2) signed_rows_kernel(
     double low[SPW];
 #pragma unroll
     for (int s = 0; s < SPW; ++s) {
-      low[s] = 0.0;  // at most 2^(M / 32) per lane; log 2 taken out exactly
+      low[s] = 0.0;  // prod is at most 2^units; log 2 taken out exactly
       if (OUT == ROWS_LOGPSI) acc[s] = two_sum(acc[s], log(ldexp(prod[s], -units)), low[s]);
     }
     if (rank == 0)
