@@ -213,12 +213,10 @@ class MetropolisSampler:
         return state
 
     def _restart(self, state):
-        """``reset`` of an existing state without the log-probabilities, which a
-        sampling call that follows writes for its own final configurations."""
+        """``reset`` of an existing state without the log-probabilities."""
         if self.reset_chains:
             state.σ = self.hilbert.random_state(state.seed, self.n_chains,
                                                 stream_id=2 + state.counter)
-        state.log_prob = torch.empty_like(state.log_prob)
         state.n_accepted_proc = torch.zeros_like(state.n_accepted_proc)
         state.n_steps_proc = 0
         return state

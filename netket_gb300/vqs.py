@@ -241,14 +241,27 @@ class MCState:
                             else int(math.ceil(n_samples / self.sampler.n_chains)))
         nd = self.n_discard_per_chain if n_discard_per_chain is None else int(n_discard_per_chain)
         p = self.params_c
-        # sampling writes the chains' log-probabilities anyway: a forward pass over
-        # them here (0.31 ms at N = 64, M = 128, 1,024 chains in FP64) would be lost
-        if type(self.sampler).reset is MetropolisSampler.reset:
-            self.sampler_state = self.sampler._restart(self.sampler_state)
+        sampler = self.sampler
+        # This library's sampling writes the chains' log-probabilities whatever they were: a
+        # forward pass over them here (0.31 ms at N = 64, M = 128, 1,024 chains in FP64) would
+        # be lost.  A sampler with a method of its own gets them, and so does the state that
+        # a refused call leaves behind.
+        own = (getattr(sampler.reset, "__func__", None) is MetropolisSampler.reset
+               and getattr(sampler.sample, "__func__", None) is MetropolisSampler.sample)
+        if own:
+            state = sampler._restart(self.sampler_state)
+            log_prob, state.log_prob = state.log_prob, torch.empty_like(state.log_prob)
         else:
-            self.sampler_state = self.sampler.reset(self.model, p, self.sampler_state)
-        self._samples, self.sampler_state = self.sampler.sample(
-            self.model, p, state=self.sampler_state, chain_length=chain_length, n_discard=nd)
+            state = sampler.reset(self.model, p, self.sampler_state)
+        self.sampler_state = state
+        try:
+            self._samples, self.sampler_state = sampler.sample(
+                self.model, p, state=state, chain_length=chain_length, n_discard=nd)
+        except BaseException:
+            if own:
+                state.log_prob = log_prob
+                sampler.reset(self.model, p, state)
+            raise
         self._cache = None
         return self._samples
 
