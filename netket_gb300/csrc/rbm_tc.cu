@@ -163,6 +163,22 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
+// e^c for 0 <= c <= 10: 2^f of the fraction f of c log2(e), 2^n by the exponent.  (The whole
+// as the argument of ex2.approx is off by up to 2e-8 in the mean, which adds up over the
+// hidden units; 2^f by about 5e-9, and 7e-9 c of the argument's low part 1.93e-8 c are left
+// out against that.)
+__device__ __forceinline__ float exp_positive(float c) {
+  constexpr float whole = 12582912.0f;  // 3 2^22: a sum has no fraction, and n in its low bits
+  const float t = __fmaf_rz(c, 1.442695022f, whole);
+  const float f = fmaf(c, 1.2e-8f, fmaf(c, 1.442695022f, whole - t));
+  return __int_as_float(__float_as_int(ex2_approx(f)) + (__float_as_int(t) << 23));
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // x_hi[s np + i] = x_si (exact), zero for i in [N, np); x_lo = 0.
 // (A warp per sample, eight sites per lane: 12.5 -> 4 us at n = 16,384, N = 256)
 __global__ void __launch_bounds__(256) spins_f16_kernel(const int8_t *__restrict__ x, int64_t n,
@@ -183,11 +199,17 @@ __global__ void __launch_bounds__(256) spins_f16_kernel(const int8_t *__restrict
   }
 }
 
-// theta += b; logpsi = sum_j log_cosh(theta_j) + a.x without tanh: the logarithm of a
-// product of cosh over eight hidden units of a lane (|theta| beyond 10 adds to the sum:
-// cosh(10 + d) = cosh(10) e^d to 2e-9), so that a unit takes two exponentials of the MUFU
-// and about ten instructions where log_cosh takes 40.  VEC: four neighbours per lane.
-// n = 16,384, M = 2,048: 55 -> 32 us (134 MB of theta: 20 us).
+// theta += b; logpsi = sum_j log_cosh(theta_j) + a.x without tanh: one log1p for eight
+// hidden units of a lane, of prod cosh - 1 (|theta| beyond 10 adds to the sum: cosh(10 + d) =
+// cosh(10) e^d to 2e-9), so that a unit takes two operations of the MUFU and about 17
+// instructions where log_cosh takes 40.  Small theta keep their precision: cosh - 1 = (E - 1)^2
+// / (2 E), E = e^|theta|, whose error is |theta| times E's, and r = prod - 1 takes a factor 1 + q
+// as r + q + r q.  (A product of cosh and its lg2.approx were off by 2^-22 per lane, more than
+// the sum at weights of 0.01.)  VEC: four neighbours per lane.
+// n = 16,384, M = 2,048: 37 us, 55 with a log_cosh per unit, 32 with the product of cosh (134
+// MB of theta: 20 us).  Error of log psi against 64 bits, rms, over that of FP32 sums of
+// log_cosh on the CUDA cores: 0.05 to 0.65 for N = 8 .. 256, M = N .. 8 N, weights of 0.01 to 1
+// (the product of cosh: 0.4 to 2.0).
 template <bool VEC>
 __global__ void __launch_bounds__(256) logpsi_cosh_kernel(
     const float *__restrict__ b, const float *__restrict__ a, const int8_t *__restrict__ x, int N,
@@ -199,7 +221,7 @@ __global__ void __launch_bounds__(256) logpsi_cosh_kernel(
   float *row = acc + s * M;
   float over = 0.0f, lg = 0.0f;
   for (int j0 = 0; j0 < M; j0 += 32 * UNITS) {
-    float th[UNITS], p = 1.0f;
+    float th[UNITS], r = 0.0f;
 #pragma unroll
     for (int k = 0; k < UNITS; k += W) {
       const int j = j0 + 32 * k + W * lane;
@@ -224,13 +246,15 @@ __global__ void __launch_bounds__(256) logpsi_cosh_kernel(
     for (int k = 0; k < UNITS; ++k) {  // (units past M: cosh 0 = 1)
       const float m = fabsf(th[k]), c = fminf(m, 10.0f);
       over += m - c;
-      p *= 0.5f * (ex2_approx(1.442695041f * c) + ex2_approx(-1.442695041f * c));
+      const float e = exp_positive(c), d = e - 1.0f;
+      const float q = 0.5f * d * (d * rcp_approx(e));
+      r = fmaf(r, q, r + q);
     }
-    lg += __log2f(p);  // at most 2^108
+    lg += log1pf(r);  // r is at most 2^108
   }
   float v = 0.0f;
   for (int i = lane; i < N; i += 32) v += (float)x[s * N + i] * a[i];
-  const float sum = warp_sum(over + 0.693147181f * lg + v);
+  const float sum = warp_sum(over + lg + v);
   if (lane == 0) logpsi[s] = sum;
 }
 
