@@ -11,7 +11,9 @@ import numpy as np
 import torch
 
 from . import _native as nat
-from .kernels import rbm_forward
+from .kernels import _use_tc, rbm_forward
+
+APPLY_ENTRIES = 1 << 28  # entries (4 bytes) of theta and the spins that apply holds at once
 
 
 def _real_param_dtype(dt):
@@ -121,8 +123,14 @@ class RBM:
         x2 = x.reshape(-1, N).contiguous()
         # large FP32 batches: x W on the tensor cores, as in every other forward pass
         # (16,384 states, N = 256, M = 2,048: 1.22 -> 0.11 ms,
-        # error against 64 bits 8e-8 -> 3.4e-8)
-        out, _, _ = rbm_forward(p, x2, N, M)
+        # error against 64 bits 8e-8 -> 3.4e-8).  That forms theta: at most 1 GiB at a time.
+        n, rows = x2.shape[0], max(1, APPLY_ENTRIES // (M + N))
+        tc = _use_tc(dtype, n, M, None)
+        if not tc or n <= rows:
+            out, _, _ = rbm_forward(p, x2, N, M)
+        else:
+            out = torch.cat([rbm_forward(p, part, N, M, use_tc=True)[0]
+                             for part in x2.split(rows)])
         return out.reshape(x.shape[:-1])
 
     def __repr__(self):
