@@ -7,18 +7,25 @@
 //   D_d = sum_{a + b = d} q_a q_b^T.
 // An entry of D_d is an integer of at most (d + 1) K 4096 <= 2^24 for K <= 512, so
 // the tensor core forms it exactly in its FP32 accumulator, whatever the order and
-// rounding of its additions.  Diagonals d = 0 .. 7 are kept (36 products); the rest
-// is below 2^-56 per term, less than the rounding of an FP64 sum.  The eight
-// integers of an entry are added in two 64-bit integers (more than 512 hidden
-// units: chunk by chunk) and only the assembly (x . x', g, 1 / n) is FP64.
+// rounding of its additions.  Diagonals d = 0 .. 7 are kept (36 products), and of
+// d = 8 the squares: where two rows are equal (on the matrix diagonal, and for a
+// configuration that was sampled twice) q_4 q_4 is positive, 2^-57.6 per hidden unit
+// in the mean, which showed at |t| = 0.03 and below (N = 16, M = 64, weights of 0.01: T's
+// diagonal off by 6.2e-16 of its largest, 3.6e-16 by FP64 sums, 3.3e-16 with the squares), while
+// the other products of d = 8 change sign.  They join D_7 as (q_4 2^-7) q_4^T, a ninth
+// operand plane (with its fractions D_7 may be rounded to 24 bits, a unit of 2^-61 at most per
+// MMA).  What is left out is at most 6.1 2^-56 per hidden unit, about 2^-56
+// sqrt(hidden units) in a sum.  The eight integers of an entry are added in two 64-bit
+// integers (more than 512 hidden units: chunk by chunk) and only the assembly
+// (x . x', g, 1 / n) is FP64.
 //
 // The FP64 pipe (two operations per clock and SM) bounded the plain form:
-// n = 4,096, M = 400: 5.74 -> 0.38 ms (digits 0.012 of it).
+// n = 4,096, M = 400: 5.74 -> 0.41 ms (digits 0.012 of it; 0.38 without the ninth plane).
 //
 // Kernel: persistent, warp-specialised (TMA warp, MMA warp, 16 epilogue warps),
 // tiles of 128 rows x 64 columns of the lower triangle.  The eight diagonals fill
-// tensor memory (8 x 64 columns); a stage holds all eight digits of 32 hidden units
-// (64-byte swizzle; A 64 KB, B 32 KB; two stages) for the 72 MMAs that use it.  The
+// tensor memory (8 x 64 columns); a stage holds all planes of 32 hidden units
+// (64-byte swizzle; A 72 KB, B 32 KB; two stages) for the 74 MMAs that use it.  The
 // epilogue empties tensor memory into registers first, so its FP64 arithmetic and
 // stores overlap the next tile's MMAs.  Waits are bounded by the library's wait
 // limit (VMCK_DEV_TIMEOUT).
@@ -33,10 +40,10 @@ namespace vmck {
 
 namespace {
 
-constexpr int H_DIGITS = 8;
+constexpr int H_DIGITS = 8, H_PLANES = H_DIGITS + 1;  // + q_4 2^-7
 constexpr int H_BM = 128, H_BN = 64, H_BK = 32, H_STAGES = 2;
 constexpr int H_A_BYTES = H_BM * H_BK * 2, H_B_BYTES = H_BN * H_BK * 2;  // one digit
-constexpr int H_STAGE_BYTES = H_DIGITS * (H_A_BYTES + H_B_BYTES);
+constexpr int H_STAGE_BYTES = H_PLANES * H_A_BYTES + H_DIGITS * H_B_BYTES;
 constexpr int H_EPI_WARPS = 16, H_THREADS = 32 * (2 + H_EPI_WARPS);
 constexpr int H_COLS = H_BN / 4;  // columns per epilogue warp (four per lane quarter)
 constexpr int H_TMEM = H_DIGITS * H_BN;
@@ -78,7 +85,7 @@ __device__ __forceinline__ void gram64_tile(int64_t t, int &I, int &J) {
   J = (int)(t - i * (i + 1));
 }
 
-// digits[a][row][k] of t, zero for k in [M, ldk); *flag is set where |t| > 1 or NaN.
+// digits[a][row][k] of t and the ninth plane, zero for k in [M, ldk); *flag is set where |t| > 1 or NaN.
 // Two neighbouring k per thread.
 __global__ void __launch_bounds__(256) gram64_digits_kernel(const double *__restrict__ t,
                                                             int64_t n, int M, int ldk,
@@ -111,6 +118,7 @@ __global__ void __launch_bounds__(256) gram64_digits_kernel(const double *__rest
 #pragma unroll
   for (int a = 0; a < H_DIGITS; ++a)
     digits[a * n * half_ld + e] = __floats2half2_rn(d[0][a], d[1][a]);
+  digits[H_DIGITS * n * half_ld + e] = __floats2half2_rn(0x1p-7f * d[0][4], 0x1p-7f * d[1][4]);
 }
 
 __global__ void __launch_bounds__(H_THREADS, 1)
@@ -181,12 +189,12 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           if (*abort_flag) break;
           unsigned char *st = smem + s * H_STAGE_BYTES;
           mbar_expect_tx(&full[s], H_STAGE_BYTES);
-          for (int a = 0; a < H_DIGITS; ++a) {
+          for (int a = 0; a < H_PLANES; ++a)
             tma_load_2d(st + a * H_A_BYTES, &mA, &full[s], kb * H_BK,
                         (int)(a * g.n) + I * H_BM);
-            tma_load_2d(st + H_DIGITS * H_A_BYTES + a * H_B_BYTES, &mB, &full[s], kb * H_BK,
+          for (int a = 0; a < H_DIGITS; ++a)
+            tma_load_2d(st + H_PLANES * H_A_BYTES + a * H_B_BYTES, &mB, &full[s], kb * H_BK,
                         (int)(a * g.n) + J * H_BN);
-          }
         }
       }
       // every copy issued must land before the CTA may exit
@@ -217,7 +225,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t a0 = smem_u32(smem + s * H_STAGE_BYTES);
-          const uint32_t b0 = a0 + H_DIGITS * H_A_BYTES;
+          const uint32_t b0 = a0 + H_PLANES * H_A_BYTES;
 #pragma unroll 1
           for (int d = 0; d < H_DIGITS; ++d) {
             const uint32_t dst = tmem_base + d * H_BN;
@@ -230,6 +238,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
                          (in_chunk == 0 && a == 0 && k == 0) ? 0u : 1u);
             }
           }
+#pragma unroll
+          for (int k = 0; k < H_BK / 16; ++k)  // (q_4 2^-7) q_4^T
+            umma_f16(tmem_base + (H_DIGITS - 1) * H_BN,
+                     umma_desc_sw64(a0 + H_DIGITS * H_A_BYTES + 32 * k),
+                     umma_desc_sw64(b0 + 4 * H_B_BYTES + 32 * k), idesc, 1u);
           umma_commit(&empty[s]);
           issued_any = true;
           if (in_chunk == H_CHUNK - 1 || kb == num_kb - 1) {
@@ -349,7 +362,7 @@ int digits_map(CUtensorMap *map, const __half *base, int64_t ldk, int64_t rows, 
 
 // Bytes: the digits (1,024-byte aligned) and the range flag.
 int64_t gram64_tc_workspace_doubles(int M, int64_t n) {
-  return (H_DIGITS * n * digits_ld(M) * 2 + 1024 + 64) / 8 + 1;
+  return (H_PLANES * n * digits_ld(M) * 2 + 1024 + 64) / 8 + 1;
 }
 
 // The plain kernel's time is its M steps of one 64 x 64 tile until the tiles fill the
@@ -359,7 +372,7 @@ int64_t gram64_tc_workspace_doubles(int M, int64_t n) {
 // n = 4,096: 609 / 5,979.
 bool gram64_tc_takes(int M, int64_t n) {
   // rows of all digits are TMA coordinates (32-bit)
-  return (M > 32 || n >= 1536) && H_DIGITS * n + H_BM < (1ll << 31);
+  return (M > 32 || n >= 1536) && H_PLANES * n + H_BM < (1ll << 31);
 }
 
 // *flag_out: device word, nonzero after the launch where t was out of range (the
@@ -381,7 +394,7 @@ int gram64_tc_launch(cudaStream_t st, const double *t, const uint32_t *bits, int
   int rc = check_launch("gram digits");
   if (rc) return rc;
   CUtensorMap mA, mB;
-  if ((rc = digits_map(&mA, digits, ldk, H_DIGITS * n, H_BM))) return rc;
+  if ((rc = digits_map(&mA, digits, ldk, H_PLANES * n, H_BM))) return rc;
   if ((rc = digits_map(&mB, digits, ldk, H_DIGITS * n, H_BN))) return rc;
   const int64_t row_tiles = (n + H_BM - 1) / H_BM;
   Gram64Params p{bits, g,  c, T64, T32,  inv_n,  shift,           n,
