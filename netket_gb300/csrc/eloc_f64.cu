@@ -14,14 +14,16 @@
 // ones.  So the factors of one- and two-site flips, divided by 1 + rho, are formed in
 // 64-bit fixed point: p + q u with p = 1 / (1 + rho) and q = 1 - p in units of 2^-63
 // and u = e^(-2 delta) < 8 in units of 2^-60, and so is their product over a lane's
-// hidden units, in units of 2^-(62 - S) where 2^S bounds it (S from the sums of |4 W|
+// hidden units, in units of 2^-(63 - S) where 2^S bounds it (S from the sums of |4 W|
 // of the row, at most 8): about 24 integer instructions where FP64 takes two operations
-// of 16 clocks per warp.  Roundings are below FP64's: 2^-60 in a factor (2^-56 for two
-// sites) and 2^-(63 - S) in a product, which is 1 or so.  A lane's product is
-// scaled anew every eight (four, two) factors, as its bound asks, and the lanes' products
-// meet as 64-bit floating-point numbers in integer registers; rows with an entry |W| >=
-// 0.52, and samples whose theta is not finite, take the FP64 form.  theta and q come from
-// integer sums too (theta_q_f64).
+// of 16 clocks per warp.  A factor is off by 2^-60 (2^-56 for two sites), a product by
+// less than a unit without a preferred sign (times_factor): below FP64's roundings while the
+// lane's product is about 1, as it is for weights of either sign.  It can fall to 2^-S,
+// where a unit is 2^-(63 - 2 S) of it: 2^-47 at S = 8, eight hidden units that all pull one
+// way.  A lane's product is scaled anew every eight (four, two) factors, as its bound asks,
+// and the lanes' products meet as 64-bit floating-point numbers in integer registers.
+// Rows with an entry |W| >= 0.52, and samples whose theta is not finite, take the FP64
+// form.  theta and q come from integer sums too (theta_q_f64).
 //
 // A product leaves the double range only where the ratio, or a partial product
 // of it, does; such an element is formed again as the difference of log_cosh sums
@@ -225,33 +227,37 @@ __device__ __forceinline__ u64 factor(u64 q, u64 u, u64 p) {
   const u64 h = mul_high(q, u, below);
   return B == 60 ? h + p : h + p + (below >> 31);
 }
-// f g for f in any units and g in units of 2^-(B - 1); f g < 2^63 units, g < 2^62 units
+// f g for f in any units and g in units of 2^-(B - 1); f < 2^63 units, f g < 2^64 units, g <
+// 2^62 units.  The result is truncated and its last bit set (odd = 1): off by less than a
+// unit, and by nothing in the mean.  A lane's first product needs neither (odd = 0): f is a
+// power of two.  (A correction after the last factor for the half units that the factors
+// before it lose is wrong by the later factors: 8e-14 of an energy where the hidden units of a
+// lane all pull one way.  Nearest rounding, an addition with carry, takes 2 to 4 % of a
+// case's time, this 1 %.)
 template <int B>
-__device__ __forceinline__ u64 times_factor(u64 f, u64 g) {
+__device__ __forceinline__ u64 times_factor(u64 f, u64 g, uint32_t odd) {
   uint32_t below;
   const u64 h = mul_high(f, g, below);
   constexpr int s = 65 - B;
   const uint32_t lo = (uint32_t)h, hi = (uint32_t)(h >> 32);
-  return (u64)__funnelshift_l(lo, hi, s) << 32 | __funnelshift_l(below, lo, s);
+  return (u64)__funnelshift_l(lo, hi, s) << 32 | (__funnelshift_l(below, lo, s) | odd);
 }
-// A lane's product: f 2^e, f within 2^(62 - 2 s) and 2^62 (s as in FlipTables' bound).
+// A lane's product: f 2^e, f within 2^(63 - 2 s) and 2^63 (s as in FlipTables' bound).
 struct LaneProduct {
   u64 f;
   int e;
 };
-__device__ __forceinline__ LaneProduct lane_one(int s) { return {1ull << (62 - s), s - 62}; }
-// after `count` factors, which lost half a unit each
-__device__ __forceinline__ UFloat lane_value(LaneProduct p, int count) {
-  return ufloat(p.f + (u64)(count >> 1), p.e);
-}
+__device__ __forceinline__ LaneProduct lane_one(int s) { return {1ull << (63 - s), s - 63}; }
+__device__ __forceinline__ UFloat lane_value(LaneProduct p) { return ufloat(p.f, p.e); }
 // ready for further factors
-__device__ __forceinline__ LaneProduct lane_renew(LaneProduct p, int count, int s) {
-  const UFloat v = lane_value(p, count);
-  return {v.m >> (s + 1), v.e + s + 1};
+__device__ __forceinline__ LaneProduct lane_renew(LaneProduct p, int s) {
+  const UFloat v = lane_value(p);
+  return {v.m >> s, v.e + s};
 }
-// Factors until lane_renew and S of rows with the summed bounds s8, s4, s2; 0: FP64 form
+// Factors until lane_renew and S of rows with the summed bounds s8, s4, s2 (S >= 1 also for
+// elements that change no site: f stays below 2^63); 0: FP64 form
 __device__ __forceinline__ int fold_length(int s8, int s4, int s2, int &s) {
-  s = s8 <= EF_S_MAX ? s8 : s4 <= EF_S_MAX ? s4 : s2;
+  s = max(1, s8 <= EF_S_MAX ? s8 : s4 <= EF_S_MAX ? s4 : s2);
   return s8 <= EF_S_MAX ? 8 : s4 <= EF_S_MAX ? 4 : s2 <= EF_S_MAX ? 2 : 0;
 }
 
@@ -344,7 +350,6 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
         }
         if (fold) fold = fold_length(S8, S4, S2, range);
         LaneProduct g[2][4 * W4];
-        int count = 0;
         if (fold) {
           const u64 offset = p_offset<60>(lane);
 #pragma unroll
@@ -358,12 +363,12 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
 #pragma unroll
               for (int t = 0; t < 2; ++t)
 #pragma unroll
-                for (int s = 0; s < S; ++s) g[t][s] = lane_renew(g[t][s], count, range);
+                for (int s = 0; s < S; ++s) g[t][s] = lane_renew(g[t][s], range);
             }
             const int je = min(M, js + 32 * fold);
-            count = (je - js - lane + 31) >> 5;
 #pragma unroll 1
             for (int j = js + lane; j < je; j += 32) {
+              const uint32_t odd = j >= 32;
               u64 u[2][2];
 #pragma unroll
               for (int t = 0; t < 2; ++t) {
@@ -376,7 +381,7 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                   const u64 ut = (bits[t] >> s) & 1 ? u[t][1] : u[t][0];
-                  g[t][s].f = times_factor<60>(g[t][s].f, factor<60>(q, ut, p));
+                  g[t][s].f = times_factor<60>(g[t][s].f, factor<60>(q, ut, p), odd);
                 }
               }
             }
@@ -406,7 +411,7 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
             if (fold) {
               UFloat quad[4];
 #pragma unroll
-              for (int s = 0; s < 4; ++s) quad[s] = lane_value(g[t][4 * w + s], count);
+              for (int s = 0; s < 4; ++s) quad[s] = lane_value(g[t][4 * w + s]);
               ok = to_double(warp_prod4(quad), r);
             } else {
               const double quad[4] = {ft[4 * w], ft[4 * w + 1], ft[4 * w + 2], ft[4 * w + 3]};
@@ -538,19 +543,18 @@ __global__ void __launch_bounds__(EF_THREADS) eloc_local_f64_kernel(
         constexpr int B = NS == 1 ? 60 : 56;  // units of an element's u
         const u64 offset = p_offset<B>(lane);
         LaneProduct g[4];
-        int count = 0;  // factors since g was scaled
 #pragma unroll
         for (int e = 0; e < 4; ++e) g[e] = lane_one(range);
 #pragma unroll 1
         for (int js = 0; js < M; js += 32 * fold) {
           if (js > 0) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) g[e] = lane_renew(g[e], count, range);
+            for (int e = 0; e < 4; ++e) g[e] = lane_renew(g[e], range);
           }
           const int je = min(M, js + 32 * fold);
-          count = (je - js - lane + 31) >> 5;
 #pragma unroll 2
           for (int j = js + lane; j < je; j += 32) {
+            const uint32_t odd = j >= 32;
             u64 u[4][NS];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
@@ -565,13 +569,13 @@ __global__ void __launch_bounds__(EF_THREADS) eloc_local_f64_kernel(
                 ue = mul_high(ue, u[e][NS - 1], below);
                 ue += below >> 31;
               }
-              g[e].f = times_factor<B>(g[e].f, factor<B>(q, ue, p));
+              g[e].f = times_factor<B>(g[e].f, factor<B>(q, ue, p), odd);
             }
           }
         }
         UFloat quad[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) quad[e] = lane_value(g[e], count);
+        for (int e = 0; e < 4; ++e) quad[e] = lane_value(g[e]);
         ok = to_double(warp_prod4(quad), r);
       } else {
         double f[4];
