@@ -22,8 +22,11 @@
 // where a unit is 2^-(63 - 2 S) of it: 2^-47 at S = 8, eight hidden units that all pull one
 // way.  A lane's product is scaled anew every eight (four, two) factors, as its bound asks,
 // and the lanes' products meet as 64-bit floating-point numbers in integer registers.
-// Rows with an entry |W| >= 0.52, and samples whose theta is not finite, take the FP64
-// form.  theta and q come from integer sums too (theta_q_f64).
+// Error of an energy, rms (one log_cosh per hidden unit and flip before), N = 16 .. 100, M =
+// 16 .. 256: weights of 0.01 to 0.1 7e-17 to 6e-16 (2e-16 to 1.4e-15); all weights of one
+// sign, 0.05 to 0.25, hidden biases of -3, 0 and 3 at most 1.5e-15 (6.7e-15).  Rows with an
+// entry |W| >= 0.52, and samples whose theta is not finite, take the FP64 form.  theta and q
+// come from integer sums too (theta_q_f64).
 //
 // A product leaves the double range only where the ratio, or a partial product
 // of it, does; such an element is formed again as the difference of log_cosh sums
@@ -80,13 +83,14 @@ __host__ __device__ inline FlipTables flip_tables(double *ws, int N, int M, int6
 // eight factors that a lane multiplies
 __global__ void __launch_bounds__(256) flip_tables_kernel(const double *__restrict__ params, int N,
                                                           int M, double *__restrict__ ws) {
-  __shared__ double red[8];
   __shared__ float size[8][32];
+  __shared__ uint32_t largest[8];
+  __shared__ long long part[2][8];
   const int64_t w = (int64_t)(N + 1) * M;
   const FlipTables tab = flip_tables(ws, N, M, 0);
   const int i = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const double *row = params + M + (int64_t)i * M;
-  double sum = 0.0;
+  uint32_t most = 0u;  // size of the row's largest entry
   float s8 = 0.0f, s4 = 0.0f, s2 = 0.0f;
   bool fits = true;
   for (int j0 = 0; j0 < M; j0 += 256) {
@@ -99,7 +103,7 @@ __global__ void __launch_bounds__(256) flip_tables_kernel(const double *__restri
       fits &= u < 8.0 && d < 8.0;
       const_cast<u64 *>(tab.uup)[(int64_t)i * M + j] = __double2ull_rn(u * 0x1p60);
       const_cast<u64 *>(tab.udown)[(int64_t)i * M + j] = __double2ull_rn(d * 0x1p60);
-      sum += v;
+      most = max(most, size_word(v));
     }
     size[warp][lane] = 5.7708f * fabsf((float)v);  // 4 |W| log2 e, rounded up
     __syncthreads();
@@ -115,6 +119,8 @@ __global__ void __launch_bounds__(256) flip_tables_kernel(const double *__restri
     }
     __syncthreads();
   }
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (lane == 0) largest[warp] = most;
   fits = __syncthreads_and(fits);
   if (warp == 0) {
     // (a small margin for the rounding of the sums)
@@ -127,12 +133,55 @@ __global__ void __launch_bounds__(256) flip_tables_kernel(const double *__restri
     if (i == N) b = make_uchar4(0, 0, 0, 0);
     if (lane == 0) const_cast<uchar4 *>(tab.bound)[i] = b;
   }
-  sum = block_sum(sum, red);
-  if (threadIdx.x == 0 && i < N) {
-    const double v = 2.0 * (sum + params[M + (int64_t)N * M + i]);
-    ws[4 * w + i] = exp(v);
-    ws[4 * w + N + i] = exp(-v);
+  if (i == N) return;
+  // The row's sum can be far beyond the log-ratios that it is part of (entries of one sign),
+  // and its exponential takes its absolute error.  Where it may be (up to 1 the exponential's
+  // own rounding is more): an integer sum as in signed_rows_kernel, and one of what its
+  // roundings leave (half a unit up in a tie, M times with one sign).
+#pragma unroll
+  for (int k = 0; k < 8; ++k) most = max(most, largest[k]);
+  const int e = most >> 20, bits = sum_bits(M);
+  const bool whole = exponent_fits(e) && (double)M * __hiloint2double((int)most, 0) > 1.0;
+  const double unit = unit_of(e, bits);
+  long long units[2] = {0, 0};
+  double plain = 0.0;
+  for (int j = threadIdx.x; j < M; j += 256) {
+    if (whole) {
+      const long long q = to_units(row[j], e, bits);
+      units[0] += q;
+      units[1] += to_units(fma((double)q, -unit, row[j]), e - bits, bits);
+    } else {
+      plain += row[j];
+    }
   }
+  if (whole) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) units[k] += __shfl_xor_sync(0xffffffffu, units[k], o);
+  } else {
+    units[0] = __double_as_longlong(warp_sum(plain));
+  }
+  if (lane < 2) part[lane][warp] = lane ? units[1] : units[0];
+  __syncthreads();
+  if (threadIdx.x > 0) return;
+  double sum = 0.0, low = 0.0;  // the second: what the first leaves
+  const double a = params[M + (int64_t)N * M + i];
+  if (whole) {
+    for (int k = 1; k < 8; ++k) {
+      units[0] += part[0][k];
+      units[1] += part[1][k];
+    }
+    sum = (double)units[0];
+    low = (double)(units[0] - (long long)sum) * unit + (double)units[1] * unit_of(e - bits, bits);
+    sum = two_sum(sum * unit, a, low);
+  } else {
+    for (int k = 0; k < 8; ++k) sum += __longlong_as_double(part[0][k]);
+    sum += a;
+  }
+  const double up = exp(2.0 * sum), down = exp(-2.0 * sum);
+  ws[4 * w + i] = fma(up, 2.0 * low, up);
+  ws[4 * w + N + i] = fma(down, -2.0 * low, down);
 }
 
 // x * W without a conversion of x: the sign bit of W flipped where x = -1

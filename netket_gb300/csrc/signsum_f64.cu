@@ -88,14 +88,6 @@ __device__ __forceinline__ void fill_table(T *tab, T w0, T w1, T w2, T w3) {
   tab[15 * 32] = -ps;
 }
 
-// a + b, its rounding error added to low (infinities and NaN reach the sum alone)
-__device__ __forceinline__ double two_sum(double a, double b, double &low) {
-  const double s = a + b, v = s - a;
-  const double e = (a - (s - v)) + (b - v);
-  if (isfinite(s)) low += e;
-  return s;
-}
-
 enum RowsOut { ROWS_LOGPSI = 0, ROWS_DOT = 1, ROWS_THETA = 2 };
 
 // A cluster takes SR_WARPS * SPW samples; its CTAs share the tiles of 32 hidden units

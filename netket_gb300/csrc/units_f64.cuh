@@ -42,6 +42,14 @@ __host__ __device__ __forceinline__ int sum_bits(int64_t terms) {
   return b;
 }
 
+// a + b, its rounding error added to low (infinities and NaN reach the sum alone)
+__device__ __forceinline__ double two_sum(double a, double b, double &low) {
+  const double s = a + b, v = s - a;
+  const double e = (a - (s - v)) + (b - v);
+  if (isfinite(s)) low += e;
+  return s;
+}
+
 // a b / 2^64 for a, b <= 2^63; below = the 32 bits under it.  (The products that a
 // 64-bit addend would carry into are written out: the compiler's own sequence takes
 // twice the instructions.)

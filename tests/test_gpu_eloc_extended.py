@@ -1,5 +1,7 @@
 """FP64 local energies (eloc_f64.cu) against extended precision where the table form loses
-most: weights of one sign, for which a lane's product moves far from 1.
+most: weights of one sign, for which a lane's product moves far from 1 and the flipped row's
+sum of weights far beyond the log-ratio (up to 150: from about 300 on, e^(2 sum) leaves the
+double range and the log_cosh route takes over).
 
 Tolerance: six times the rms of independent roundings.  With a = 4 |W| log2 e of eight
 neighbours' sum S <= 8, a lane's product of eight factors in units of 2^-(63 - S) is off by at
@@ -39,7 +41,7 @@ def _energies(flat, x, N, M):
 
 @pytest.mark.parametrize("N,M,weight,bias", [
     (16, 512, 0.13, 3.0), (16, 512, 0.13, 0.0), (16, 512, 0.13, -3.0), (64, 256, 0.13, 3.0),
-    (64, 256, 0.1, -3.0), (12, 264, 0.09, 3.0)])
+    (64, 256, 0.1, -3.0), (12, 264, 0.09, 3.0), (6, 3000, 0.05, 0.0), (6, 2500, 0.06, 2.0)])
 def test_weights_of_one_sign(N, M, weight, bias):
     n = 24
     g = np.random.default_rng(N + M)
