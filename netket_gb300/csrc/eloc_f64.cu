@@ -256,6 +256,12 @@ __device__ __forceinline__ bool to_double(UFloat v, double &d) {
   return v.e > -1000 && v.e < 890;
 }
 
+// e^(-2 theta), and NaN for an infinite theta: its sample's products then take the log_cosh
+// route, where the ratio is a difference of infinities.
+__device__ __forceinline__ double rho_of(double theta) {
+  return exp(-2.0 * theta) + (theta - theta);
+}
+
 // Product of 1 / (1 + rho_j) over the hidden units j = lane, lane + 32, ...
 __device__ __forceinline__ double lane_norm(const double *rho, int M) {
   double v = 1.0;
@@ -376,7 +382,7 @@ __global__ void __launch_bounds__(ising_threads<S>(), S == 8 ? 2 : 4) eloc_ising
       if (odd) {
         for (int s = 0; s < S; ++s)
           for (int j = tid; j < M; j += THREADS)
-            rho[s * M + j] = exp(-2.0 * tab.theta[min(b0 + s, n - 1) * M + j]);
+            rho[s * M + j] = rho_of(tab.theta[min(b0 + s, n - 1) * M + j]);
         __syncthreads();
         for (int s = warp; s < S; s += WARPS) norm[s][lane] = lane_norm(rho + s * M, M);
         __syncthreads();
@@ -538,7 +544,7 @@ __global__ void __launch_bounds__(EF_THREADS) eloc_local_f64_kernel(
     const bool fp64 = __syncthreads_or(NS > 2 || odd || !finite);
     const int kept = local_conn_enumerate(op, sh, g, true);
     if (fp64) {
-      for (int j = tid; j < M; j += EF_THREADS) rho[j] = exp(-2.0 * tab.theta[b * M + j]);
+      for (int j = tid; j < M; j += EF_THREADS) rho[j] = rho_of(tab.theta[b * M + j]);
       __syncthreads();
       if (warp == 0) norm[lane] = lane_norm(rho, M);
     }

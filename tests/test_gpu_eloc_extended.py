@@ -57,3 +57,21 @@ def test_weights_of_one_sign(N, M, weight, bias):
     tol = 6 * rms
     err = np.abs(_energies(flat, x, N, M) - (diag - flips)) / np.maximum(1, flips)
     assert err.max() <= tol
+
+
+@pytest.mark.parametrize("N,M", [(8, 40), (70, 33)])
+@pytest.mark.parametrize("bias", [np.inf, -np.inf, np.nan])
+def test_infinite_theta_gives_nan(N, M, bias):
+    """A hidden bias that is not finite: psi(x') / psi(x) is a quotient of infinities, and no
+    energy may look finite."""
+    import netket_gb300 as nk
+    g = np.random.default_rng(1)
+    flat = g.normal(size=M + N * M + N) * 0.1
+    flat[3] = bias
+    x = (2 * g.integers(0, 2, size=(40, N)) - 1).astype(np.int8)
+    x[:, :2] = 1, -1
+    assert np.isnan(_energies(flat, x, N, M)).all()
+    H = nk.operator.Heisenberg(nk.hilbert.Spin(0.5, N), nk.graph.Chain(N))
+    e = nk.kernels.local_energies_fused(H, torch.as_tensor(flat).cuda(), torch.as_tensor(x).cuda(),
+                                        N, M)
+    assert bool(torch.isnan(e).all())
