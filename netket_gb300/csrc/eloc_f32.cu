@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(WSM ? E3_GROUP *E3_MAX_GROUPS : E3_GROUP)
       for (int k = 0; k < 4; ++k) p[k] += __shfl_xor_sync(0xffffffffu, p[k], o);
     float s = (p[0] + p[2]) + (p[1] + p[3]);
     s += d0 * (WSM ? as[s0] : __ldg(a + s0));
-    if (!ISING) s += d1 * (WSM ? as[s1] : __ldg(a + s1));
+    // (a one-site element's second site is a placeholder)
+    if (!ISING && d1 != 0.0f) s += d1 * (WSM ? as[s1] : __ldg(a + s1));
     return s;
   };
 
