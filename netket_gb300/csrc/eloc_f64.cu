@@ -42,7 +42,11 @@ namespace vmck {
 constexpr int EF_THREADS = 128, EF_WARPS = EF_THREADS / 32;  // LocalOperator
 constexpr int EF_S_MAX = 8;
 constexpr int EF_DIRECT = 12;
-constexpr int64_t EF_CHUNK = 16384;  // samples whose theta and q are kept at once
+// Samples whose theta and q (16 bytes per hidden unit) are kept at once: 512 MB at most
+__host__ __device__ inline int64_t ef_chunk(int M, int64_t n) {
+  const int64_t most = M <= 2048 ? 16384 : (1ll << 25) / M;
+  return n < most ? n : (most > 0 ? most : 1);
+}
 
 // Tables of the call: up[i, j] = exp(-4 W_ij) and down[i, j] = exp(4 W_ij), the
 // factor e^(-2 delta) of turning spin i up (x = -1 -> 1) and down, for i < N and
@@ -61,7 +65,7 @@ struct FlipTables {
 };
 
 __host__ __device__ inline int64_t flip_table_len(int N, int M, int64_t n) {
-  return 4 * (int64_t)(N + 1) * M + 2 * N + (N + 2) / 2 + 2 * (n < EF_CHUNK ? n : EF_CHUNK) * M;
+  return 4 * (int64_t)(N + 1) * M + 2 * N + (N + 2) / 2 + 2 * ef_chunk(M, n) * M;
 }
 
 // n: samples of a chunk
@@ -756,7 +760,7 @@ extern "C" int vmck_rbm_eloc_ising_f64(vmck_stream s, const double *params, int3
     return vmck_rbm_eloc_ising(s, VMCK_F64, params, N, M, x, n, edges, n_edges, h, J, eloc,
                                nullptr);
   int rc;
-  const int64_t chunk = std::min(n, EF_CHUNK);
+  const int64_t chunk = ef_chunk(M, n);
   const FlipTables tab = flip_tables(workspace, N, M, chunk);
   if (h != 0.0 && (rc = launch_flip_tables(st, params, N, M, workspace))) return rc;
   for (int64_t c = 0; c < n; c += chunk, x += chunk * N, eloc += chunk) {
@@ -797,7 +801,7 @@ extern "C" int vmck_rbm_eloc_local_f64(vmck_stream s, const double *params, int3
   if (!signed_rows_fit(N))
     return vmck_rbm_eloc_local(s, VMCK_F64, params, N, M, x, n, op, eloc, nullptr);
   if ((rc = launch_flip_tables(st, params, N, M, workspace))) return rc;
-  const int64_t chunk = std::min(n, EF_CHUNK);
+  const int64_t chunk = ef_chunk(M, n);
   const FlipTables tab = flip_tables(workspace, N, M, chunk);
   for (int64_t c = 0; c < n; c += chunk, x += chunk * N, eloc += chunk) {
     const int64_t m = std::min(chunk, n - c);
