@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(256) abs_max_scale_kernel(const T *__restrict_
 
 template <typename T>
 static int launch_abs_max_scale(cudaStream_t st, const T *v, int64_t n, float *scale) {
-  // the two counters follow the scale in its workspace slot
+  // the largest |v| and the counter of finished blocks follow the scale in its workspace slot
   unsigned *words = reinterpret_cast<unsigned *>(scale + 1);
   VMCK_CUDA(cudaMemsetAsync(words, 0, 2 * sizeof(unsigned), st));
   const int64_t blocks = std::min<int64_t>((n + 2047) / 2048, 304);
@@ -210,15 +210,26 @@ __global__ void __launch_bounds__(256) spins_f16_kernel(const int8_t *__restrict
 // MB of theta: 20 us).  Error of log psi against 64 bits, rms, over that of FP32 sums of
 // log_cosh on the CUDA cores: 0.05 to 0.65 for N = 8 .. 256, M = N .. 8 N, weights of 0.01 to 1
 // (the product of cosh: 0.4 to 2.0).
+// most: the bits of the largest |W_ij|.  With an infinite weight every FP16 product of its
+// column is NaN (infinity times the spins' low part, 0); x W is then formed here.
 template <bool VEC>
 __global__ void __launch_bounds__(256) logpsi_cosh_kernel(
     const float *__restrict__ b, const float *__restrict__ a, const int8_t *__restrict__ x, int N,
-    int M, int64_t n, float *__restrict__ acc, float *__restrict__ logpsi, bool keep_theta) {
+    int M, int64_t n, float *__restrict__ acc, float *__restrict__ logpsi, bool keep_theta,
+    const float *__restrict__ weights, const unsigned *__restrict__ most) {
   constexpr int W = VEC ? 4 : 1, UNITS = 8;
   const int64_t s = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (s >= n) return;
   float *row = acc + s * M;
+  if (*most >= 0x7f800000u) {
+    for (int j = lane; j < M; j += 32) {
+      float t = 0.0f;
+      for (int i = 0; i < N; ++i) t += (float)x[s * N + i] * weights[(int64_t)i * M + j];
+      row[j] = t;
+    }
+    __syncwarp();
+  }
   float over = 0.0f, lg = 0.0f;
   for (int j0 = 0; j0 < M; j0 += 32 * UNITS) {
     float th[UNITS], r = 0.0f;
@@ -395,16 +406,17 @@ extern "C" int vmck_rbm_logpsi_tc(vmck_stream s, const float *params, int32_t N,
                     nullptr, nullptr, 0, 0, 0, nullptr, status, 0)))
     return rc;
   const bool keep = theta_out != nullptr;
+  const unsigned *most = reinterpret_cast<const unsigned *>(w.scale + 1);  // launch_abs_max_scale
   if (tanh_out)
     logpsi_epilogue_kernel<<<ceil_div(n, 8), 256, 0, st>>>(bvec, avec, x, N, M, n, acc, logpsi,
                                                            keep, tanh_out);
   else if (M % 4 == 0 && (reinterpret_cast<uintptr_t>(acc) | reinterpret_cast<uintptr_t>(bvec)) %
                                  16 == 0)
     logpsi_cosh_kernel<true><<<ceil_div(n, 8), 256, 0, st>>>(bvec, avec, x, N, M, n, acc, logpsi,
-                                                             keep);
+                                                             keep, W, most);
   else
     logpsi_cosh_kernel<false><<<ceil_div(n, 8), 256, 0, st>>>(bvec, avec, x, N, M, n, acc, logpsi,
-                                                              keep);
+                                                              keep, W, most);
   return check_launch("rbm_logpsi_tc epilogue");
 }
 
