@@ -1,23 +1,23 @@
 // T = O_L O_L^T + diag_shift I for FP64 tanh(theta), the contraction t t^T on the
 // tcgen05 tensor cores.
 //
-// t (|t| <= 1) is rounded to a multiple of 2^-55 and written in balanced base-128
-// digits, t = sum_a q_a 2^(-6 - 7 a), a = 0 .. 7, |q_a| <= 64: eight matrices of
-// small integers, exact in FP16.  t t^T is then sum_d 2^(-12 - 7 d) D_d with
+// A row of t (|t| <= 1), times the power of two that brings its largest entry to [1/2, 1), is
+// rounded to a multiple of 2^-55 and written in balanced base-128 digits, t 2^s = sum_a
+// q_a 2^(-6 - 7 a), a = 0 .. 7, |q_a| <= 64: eight matrices of small integers, exact in
+// FP16.  t t^T is then 2^(-s - s') sum_d 2^(-12 - 7 d) D_d with
 //   D_d = sum_{a + b = d} q_a q_b^T.
 // An entry of D_d is an integer of at most (d + 1) K 4096 <= 2^24 for K <= 512, so
 // the tensor core forms it exactly in its FP32 accumulator, whatever the order and
 // rounding of its additions.  Diagonals d = 0 .. 7 are kept (36 products), and of
 // d = 8 the squares: where two rows are equal (on the matrix diagonal, and for a
 // configuration that was sampled twice) q_4 q_4 is positive, 2^-57.6 per hidden unit
-// in the mean, which showed at |t| = 0.03 and below (N = 16, M = 64, weights of 0.01: T's
-// diagonal off by 6.2e-16 of its largest, 3.6e-16 by FP64 sums, 3.3e-16 with the squares), while
-// the other products of d = 8 change sign.  They join D_7 as (q_4 2^-7) q_4^T, a ninth
-// operand plane (with its fractions D_7 may be rounded to 24 bits, a unit of 2^-61 at most per
-// MMA).  What is left out is at most 6.1 2^-56 per hidden unit, about 2^-56
-// sqrt(hidden units) in a sum.  The eight integers of an entry are added in two 64-bit
-// integers (more than 512 hidden units: chunk by chunk) and only the assembly
-// (x . x', g, 1 / n) is FP64.
+// in the mean, while the other products of d = 8 change sign.  They join D_7 as
+// q_4 (q_4 2^-7)^T, a ninth operand plane (with its fractions D_7 may be rounded to 24
+// bits, a unit of 2^-61 at most per MMA).  What is left out is at most 6.1 2^-56 per hidden
+// unit, about 2^-56 sqrt(hidden units) in a sum, of the product of the rows' largest
+// entries.  Error of T, rms, over that of FP64 sums: 0.15 to 0.86 (weights of 0.001 to 0.3, N =
+// 8 .. 100, M = 32 .. 400).  The eight integers of an entry are added in two 64-bit integers
+// (more than 512 hidden units: chunk by chunk) and only the assembly (x . x', g, 1 / n) is FP64.
 //
 // The FP64 pipe (two operations per clock and SM) bounded the plain form:
 // n = 4,096, M = 400: 5.74 -> 0.41 ms (digits 0.012 of it; 0.38 without the ninth plane).
@@ -25,7 +25,7 @@
 // Kernel: persistent, warp-specialised (TMA warp, MMA warp, 16 epilogue warps),
 // tiles of 128 rows x 64 columns of the lower triangle.  The eight diagonals fill
 // tensor memory (8 x 64 columns); a stage holds all planes of 32 hidden units
-// (64-byte swizzle; A 72 KB, B 32 KB; two stages) for the 74 MMAs that use it.  The
+// (64-byte swizzle; A 64 KB, B 36 KB; two stages) for the 74 MMAs that use it.  The
 // epilogue empties tensor memory into registers first, so its FP64 arithmetic and
 // stores overlap the next tile's MMAs.  Waits are bounded by the library's wait
 // limit (VMCK_DEV_TIMEOUT).
@@ -35,6 +35,7 @@
 
 #include "gram_tc.cuh"
 #include "tc_common.cuh"
+#include "units_f64.cuh"
 
 namespace vmck {
 
@@ -43,12 +44,13 @@ namespace {
 constexpr int H_DIGITS = 8, H_PLANES = H_DIGITS + 1;  // + q_4 2^-7
 constexpr int H_BM = 128, H_BN = 64, H_BK = 32, H_STAGES = 2;
 constexpr int H_A_BYTES = H_BM * H_BK * 2, H_B_BYTES = H_BN * H_BK * 2;  // one digit
-constexpr int H_STAGE_BYTES = H_PLANES * H_A_BYTES + H_DIGITS * H_B_BYTES;
+constexpr int H_STAGE_BYTES = H_DIGITS * H_A_BYTES + H_PLANES * H_B_BYTES;
 constexpr int H_EPI_WARPS = 16, H_THREADS = 32 * (2 + H_EPI_WARPS);
 constexpr int H_COLS = H_BN / 4;  // columns per epilogue warp (four per lane quarter)
 constexpr int H_TMEM = H_DIGITS * H_BN;
 constexpr int H_CHUNK = 512 / H_BK;  // stages whose sums stay below 2^24
 constexpr int H_WORDS = 9;           // sign words of N <= 288
+constexpr int H_SHIFT_MAX = 480;     // 2^(-61 - 2 s) is a normal number
 
 // K-major operand with 64-byte swizzle: 8-row groups 512 bytes apart, layout
 // SWIZZLE_64B = 4 (fields as in umma_desc_sw128).
@@ -71,6 +73,7 @@ struct Gram64Params {
   int64_t n;
   int words, N, M;
   const int *skip;  // nonzero: t is out of range, the plain kernel forms T
+  const int *shift_of;  // s of each row
   int32_t *status;
   unsigned long long wait_ns;
   int64_t tiles;
@@ -85,40 +88,47 @@ __device__ __forceinline__ void gram64_tile(int64_t t, int &I, int &J) {
   J = (int)(t - i * (i + 1));
 }
 
-// digits[a][row][k] of t and the ninth plane, zero for k in [M, ldk); *flag is set where |t| > 1 or NaN.
-// Two neighbouring k per thread.
+// digits[a][row][k] of t 2^s and the ninth plane, zero for k in [M, ldk), and s of each row;
+// *flag is set where |t| > 1 or NaN.  A warp per row, two neighbouring k per lane.
 __global__ void __launch_bounds__(256) gram64_digits_kernel(const double *__restrict__ t,
                                                             int64_t n, int M, int ldk,
                                                             __half2 *__restrict__ digits,
+                                                            int *__restrict__ shift_of,
                                                             int *flag) {
+  const int64_t r = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= n) return;
+  const double *row = t + r * M;
+  uint32_t most = 0u;
+  for (int k = lane; k < M; k += 32) most = max(most, size_word(__ldg(row + k)));
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (most > 0x3ff00000u) {  // |t| > 1 or NaN
+    if (lane == 0) atomicOr(flag, 1);
+    return;
+  }
+  const int s = most == 0u ? 0 : min(max(1022 - (int)(most >> 20), 0), H_SHIFT_MAX);
+  if (lane == 0) shift_of[r] = s;
+  const double scale = __hiloint2double((1023 + 55 + s) << 20, 0);
   const int half_ld = ldk / 2;
-  const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (e >= n * half_ld) return;
-  const int64_t r = e / half_ld;
-  const int k = 2 * (int)(e - r * half_ld);
-  long long v[2];
+  __half2 *out = digits + r * half_ld;
+  for (int h = lane; h < half_ld; h += 32) {
+    float d[2][H_DIGITS];
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-    const double x = k + q < M ? t[r * M + k + q] : 0.0;
-    const bool ok = fabs(x) <= 1.0;
-    if (!ok) atomicOr(flag, 1);
-    v[q] = ok ? __double2ll_rn(x * 36028797018963968.0) : 0ll;  // 2^55
-  }
-  float d[2][H_DIGITS];
+    for (int q = 0; q < 2; ++q) {
+      long long v = 2 * h + q < M ? __double2ll_rn(__ldg(row + 2 * h + q) * scale) : 0ll;
 #pragma unroll
-  for (int q = 0; q < 2; ++q) {
-#pragma unroll
-    for (int a = H_DIGITS - 1; a > 0; --a) {
-      const int low = (int)((v[q] + 64) & 127) - 64;
-      d[q][a] = (float)low;
-      v[q] = (v[q] - low) >> 7;
+      for (int a = H_DIGITS - 1; a > 0; --a) {
+        const int low = (int)((v + 64) & 127) - 64;
+        d[q][a] = (float)low;
+        v = (v - low) >> 7;
+      }
+      d[q][0] = (float)(int)v;
     }
-    d[q][0] = (float)(int)v[q];
-  }
 #pragma unroll
-  for (int a = 0; a < H_DIGITS; ++a)
-    digits[a * n * half_ld + e] = __floats2half2_rn(d[0][a], d[1][a]);
-  digits[H_DIGITS * n * half_ld + e] = __floats2half2_rn(0x1p-7f * d[0][4], 0x1p-7f * d[1][4]);
+    for (int a = 0; a < H_DIGITS; ++a)
+      out[a * n * half_ld + h] = __floats2half2_rn(d[0][a], d[1][a]);
+    out[H_DIGITS * n * half_ld + h] = __floats2half2_rn(0x1p-7f * d[0][4], 0x1p-7f * d[1][4]);
+  }
 }
 
 __global__ void __launch_bounds__(H_THREADS, 1)
@@ -189,11 +199,11 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           if (*abort_flag) break;
           unsigned char *st = smem + s * H_STAGE_BYTES;
           mbar_expect_tx(&full[s], H_STAGE_BYTES);
-          for (int a = 0; a < H_PLANES; ++a)
+          for (int a = 0; a < H_DIGITS; ++a)
             tma_load_2d(st + a * H_A_BYTES, &mA, &full[s], kb * H_BK,
                         (int)(a * g.n) + I * H_BM);
-          for (int a = 0; a < H_DIGITS; ++a)
-            tma_load_2d(st + H_PLANES * H_A_BYTES + a * H_B_BYTES, &mB, &full[s], kb * H_BK,
+          for (int a = 0; a < H_PLANES; ++a)
+            tma_load_2d(st + H_DIGITS * H_A_BYTES + a * H_B_BYTES, &mB, &full[s], kb * H_BK,
                         (int)(a * g.n) + J * H_BN);
         }
       }
@@ -225,7 +235,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t a0 = smem_u32(smem + s * H_STAGE_BYTES);
-          const uint32_t b0 = a0 + H_PLANES * H_A_BYTES;
+          const uint32_t b0 = a0 + H_DIGITS * H_A_BYTES;
 #pragma unroll 1
           for (int d = 0; d < H_DIGITS; ++d) {
             const uint32_t dst = tmem_base + d * H_BN;
@@ -239,10 +249,9 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             }
           }
 #pragma unroll
-          for (int k = 0; k < H_BK / 16; ++k)  // (q_4 2^-7) q_4^T
-            umma_f16(tmem_base + (H_DIGITS - 1) * H_BN,
-                     umma_desc_sw64(a0 + H_DIGITS * H_A_BYTES + 32 * k),
-                     umma_desc_sw64(b0 + 4 * H_B_BYTES + 32 * k), idesc, 1u);
+          for (int k = 0; k < H_BK / 16; ++k)  // q_4 (q_4 2^-7)^T
+            umma_f16(tmem_base + (H_DIGITS - 1) * H_BN, umma_desc_sw64(a0 + 4 * H_A_BYTES + 32 * k),
+                     umma_desc_sw64(b0 + H_DIGITS * H_B_BYTES + 32 * k), idesc, 1u);
           umma_commit(&empty[s]);
           issued_any = true;
           if (in_chunk == H_CHUNK - 1 || kb == num_kb - 1) {
@@ -268,7 +277,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
     for (int64_t tile = blockIdx.x; tile < g.tiles && alive; tile += gridDim.x) {
       int I, J;
       gram64_tile(tile, I, J);
-      // sum_d D_d 2^(-12 - 7 d) = hi 2^-33 + lo 2^-61
+      // sum_d D_d 2^(-12 - 7 d) = hi 2^-33 + lo 2^-61 (times 2^(-s - s'))
       long long hi[H_COLS], lo[H_COLS];
 #pragma unroll
       for (int j = 0; j < H_COLS; ++j) hi[j] = lo[j] = 0;
@@ -304,6 +313,7 @@ __global__ void __launch_bounds__(H_THREADS, 1)
         for (int w = 0; w < H_WORDS; ++w)
           rb[w] = w < g.words ? __ldg(g.bits + row * g.words + w) : 0u;
         const double gr = cc - __ldg(g.g + row);
+        const int sr = 1023 - __ldg(g.shift_of + row);
         double *out = g.T64 ? g.T64 + row * g.n + col0 : nullptr;
         float *out32 = g.T32 ? g.T32 + row * g.n + col0 : nullptr;
 #pragma unroll
@@ -315,7 +325,9 @@ __global__ void __launch_bounds__(H_THREADS, 1)
             for (int w = 0; w < H_WORDS; ++w)
               if (w < g.words) diff += __popc(rb[w] ^ __ldg(g.bits + col * g.words + w));
             const int B = g.N - 2 * diff;
-            const double A = fma((double)hi[j], 0x1p-33, (double)lo[j] * 0x1p-61);
+            const int es = (sr - __ldg(g.shift_of + col)) << 20;  // exponent of 2^(-s - s')
+            const double A = fma((double)hi[j], __hiloint2double(es - (33 << 20), 0),
+                                 (double)lo[j] * __hiloint2double(es - (61 << 20), 0));
             double v = (fma(A, (double)(1 + B), (double)B) + (gr - __ldg(g.g + col))) * g.inv_n;
             if (col == row) v += g.shift;
             if (out) out[j] = v;
@@ -360,9 +372,9 @@ int digits_map(CUtensorMap *map, const __half *base, int64_t ldk, int64_t rows, 
 
 }  // namespace
 
-// Bytes: the digits (1,024-byte aligned) and the range flag.
+// Bytes: the range flag, the digits (1,024-byte aligned) and the rows' shifts.
 int64_t gram64_tc_workspace_doubles(int M, int64_t n) {
-  return (H_PLANES * n * digits_ld(M) * 2 + 1024 + 64) / 8 + 1;
+  return (H_PLANES * n * digits_ld(M) * 2 + 1024 + 64 + 4 * n) / 8 + 1;
 }
 
 // The plain kernel's time is its M steps of one 64 x 64 tile until the tiles fill the
@@ -387,18 +399,18 @@ int gram64_tc_launch(cudaStream_t st, const double *t, const uint32_t *bits, int
   *flag_out = flag;
   const int ldk = (int)digits_ld(M);
   VMCK_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
-  const int64_t pairs = n * (ldk / 2);
-  VMCK_REQUIRE((pairs + 255) / 256 < (1ll << 31), "rbm_gram: too many samples");
-  gram64_digits_kernel<<<(unsigned)((pairs + 255) / 256), 256, 0, st>>>(
-      t, n, M, ldk, reinterpret_cast<__half2 *>(digits), flag);
+  int *shift_of = reinterpret_cast<int *>(digits + H_PLANES * n * ldk);
+  gram64_digits_kernel<<<(unsigned)((n + 7) / 8), 256, 0, st>>>(
+      t, n, M, ldk, reinterpret_cast<__half2 *>(digits), shift_of, flag);
   int rc = check_launch("gram digits");
   if (rc) return rc;
   CUtensorMap mA, mB;
-  if ((rc = digits_map(&mA, digits, ldk, H_PLANES * n, H_BM))) return rc;
-  if ((rc = digits_map(&mB, digits, ldk, H_DIGITS * n, H_BN))) return rc;
+  if ((rc = digits_map(&mA, digits, ldk, H_DIGITS * n, H_BM))) return rc;
+  if ((rc = digits_map(&mB, digits, ldk, H_PLANES * n, H_BN))) return rc;
   const int64_t row_tiles = (n + H_BM - 1) / H_BM;
   Gram64Params p{bits, g,  c, T64, T32,  inv_n,  shift,           n,
-                 words, N, M, flag, status, wait_limit_ns(), row_tiles * (row_tiles + 1)};
+                 words, N, M, flag, shift_of, status, wait_limit_ns(),
+                 row_tiles * (row_tiles + 1)};
   const size_t smem = 1024 + H_STAGES * H_STAGE_BYTES + 128;
   VMCK_CUDA(cudaFuncSetAttribute(gram64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
