@@ -198,7 +198,8 @@ int vmck_rbm_eloc_local(vmck_stream s, int32_t dtype, const void *params, int32_
 /* The same in FP64 from tables of flip factors exp(+-4 W), made once per call in
  * the caller's workspace (at least vmck_rbm_eloc_f64_workspace_size(N, M, n)
  * doubles): one factor per hidden unit and connected element, in 64-bit fixed point
- * for flips of one or two sites, instead of a log_cosh. */
+ * for flips of one or two sites, instead of a log_cosh.  theta is kept of at most 16,384
+ * samples (2^25 / M beyond M = 2,048) at a time. */
 int64_t vmck_rbm_eloc_f64_workspace_size(int32_t N, int32_t M, int64_t n);
 int vmck_rbm_eloc_ising_f64(vmck_stream s, const double *params, int32_t N, int32_t M,
                             const int8_t *x, int64_t n, const int32_t *edges,
@@ -410,7 +411,8 @@ int vmck_rbm_jacobian(vmck_stream s, int32_t dtype, const void *tanh_theta,
  *   T = (G - g 1^T - 1 g^T + c 11^T) / n + diag_shift I, g = O obar, c = |obar|^2.
  * obar (P, FP64): column means.  Only the lower triangle (row >= col) is written;
  * T64 (n, n) FP64 row-major; T32 (nullable) receives an FP32 copy.
- * mode 0: FP64 contraction (CUDA cores); 1: FP32 contraction (CUDA cores);
+ * mode 0: FP64 contraction (CUDA cores, or the tensor cores by exact digit products: see
+ * vmck_gram_f64_workspace_size); 1: FP32 contraction (CUDA cores);
  * 2: tensor cores (tcgen05, TMA) on t rounded to hi + lo BF16 pairs (all four
  * products, FP32 accumulation); 3: tensor cores on t rounded to one BF16;
  * 4: tensor cores on t - fp32(tbar) rounded to a multiple of 2^-19 and split
@@ -425,8 +427,8 @@ int vmck_rbm_jacobian(vmck_stream s, int32_t dtype, const void *tanh_theta,
  * VMCK_DEV_TIMEOUT if a tensor-core CTA's bounded wait ran out. */
 int64_t vmck_gram_workspace_size(int32_t N, int32_t M, int64_t n);
 /* Mode 0 with a workspace of at least this many doubles contracts on the tensor
- * cores where that is faster: |t| <= 1 rounded to a multiple of 2^-55, in base-128
- * digits whose products sum exactly (an error below an FP64 sum's). */
+ * cores where that is faster: |t| <= 1 rounded to 2^-55 of the row's largest entry (its power
+ * of two), in base-128 digits whose products sum exactly (an error below an FP64 sum's). */
 int64_t vmck_gram_f64_workspace_size(int32_t N, int32_t M, int64_t n);
 
 int vmck_rbm_gram(vmck_ctx *ctx, vmck_stream s, int32_t mode, int32_t dtype,

@@ -30,10 +30,9 @@ constexpr int E3_GROUP = 128;       // threads of a sample's group
 constexpr int E3_MAX_GROUPS = 6;    // groups per CTA with the weights in shared memory
 constexpr size_t E3_SMEM_MAX = 227 * 1024 - 2048;
 
-// log_cosh_fast with e^(-2|x|) in one multiplication and one MUFU operation.  The
-// product is -2 |x| log2(e) rounded once, as __expf(-2 |x|) forms it; results it
-// flushes to zero (|x| > 43) are below 1e-37 and leave the polynomial at its
-// constant either way.
+// log_cosh_fast, bit for bit (test_gpu_eloc_f32.py compares the energies), with e^(-2|x|) = 2^(-2
+// |x| log2 e) in one multiplication and one MUFU operation; what the operation flushes to
+// zero (|x| > 43) is below 1e-37 and leaves the polynomial at its constant either way.
 __device__ __forceinline__ float log_cosh_ftz(float x) {
   x = fabsf(x);
   float e;

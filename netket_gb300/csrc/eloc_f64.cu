@@ -327,7 +327,7 @@ __device__ __forceinline__ int fold_length(int s8, int s4, int s2, int &s) {
 // (warp_prod4).  Lane group e accumulates sample e's (and e + 4's) sum.
 // N = 256, M = 256, n = 2,048: 0.34 ms with the tables and theta (products in FP64
 // 1.14 ms; one log_cosh per hidden unit and flip, eloc_ising_kernel<double>, 20.1 ms).
-// The issue of the integer products bounds it: 42 % of the slots at 16 warps per SM,
+// The issue of the integer products bounds it: 50 % of the slots at 16 warps per SM,
 // whatever a warp's samples and sites (four, eight; one, two).
 template <int S>
 constexpr int ising_threads() {

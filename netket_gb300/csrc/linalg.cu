@@ -1732,7 +1732,7 @@ static int refined_solve(vmck_ctx *c, cudaStream_t st, const double *A64, float 
   const int64_t np = factor_mode == 4 ? ((n + 3) & ~int64_t(3)) : n;
   const bool own_trsv = (factor_mode == 3 && n % 4 == 0) || factor_mode == 4;
   // aux: r (n double), r32 (np float), two norms + done + prev, symv slots
-  // (strips + segments rows of n double), inverse diagonal blocks (mode 3), the solves' published
+  // (a row of n double per 64-row tile), inverse diagonal blocks (mode 3), the solves' published
   // words (2 nb TB), tickets and counters (4 uint), residual check partials, leaf
   // inverses (mode 3)
   const int64_t nb = (np + TB - 1) / TB;

@@ -32,7 +32,7 @@
 //
 // Measured (GB300, MCState.sample, before -> now; before = one log_cosh per hidden
 // unit and proposal): FP64 Local, N = 64, M = 128, 1,024 chains x 9 sweeps 14.1 ->
-// 0.28 ms; FP64 Exchange, N = 36, M = 72, 1,024 chains 7.77 -> 0.23 ms; FP32
+// 0.26 ms; FP64 Exchange, N = 36, M = 72, 1,024 chains 7.77 -> 0.23 ms; FP32
 // Exchange, 10 x 10 J1-J2, M = 400, 4,096 chains 3.45 -> 1.10 ms (about 880 warp
 // instructions per proposal before, 312 now).
 #include <algorithm>
@@ -316,7 +316,10 @@ __global__ void __launch_bounds__(32 * max_warps<T, R>(), 1)
   }
 }
 
-// Registers per lane for the hidden layer: 32 R >= M.
+// Registers per lane for the hidden layer: 32 R >= M.  Thirteen beside sixteen: what a
+// proposal issues and the shared memory of a row follow R (10 x 10 J1-J2, 4,096 chains, kernel
+// time with R = 13 / 16, us: M = 400 Exchange FP32 1,089 / 1,230, FP64 2,959 / 3,382, Local 655 /
+// 772, 2,922 / 3,114; M = 260 Exchange FP64 2,729 / 3,259, Local FP32 659 / 777).
 static int filter_regs(int M) {
   for (int r : {1, 2, 4, 8, 13, 16})
     if (M <= 32 * r) return r;
