@@ -250,7 +250,8 @@ class MCState:
                and getattr(sampler.sample, "__func__", None) is MetropolisSampler.sample)
         if own:
             state = sampler._restart(self.sampler_state)
-            log_prob, state.log_prob = state.log_prob, torch.empty_like(state.log_prob)
+            log_prob, σ = state.log_prob, state.σ
+            state.log_prob = torch.empty(σ.shape[0], dtype=torch.float64, device=σ.device)
         else:
             state = sampler.reset(self.model, p, self.sampler_state)
         self.sampler_state = state

@@ -41,3 +41,14 @@ def test_a_sampler_of_its_own_gets_log_probabilities():
         assert torch.equal(log_prob, 2.0 * vs.log_value(sigma))
     st = vs.sampler_state  # and the call writes those of the final configurations
     torch.testing.assert_close(st.log_prob, 2.0 * vs.log_value(st.σ), rtol=1e-12, atol=1e-12)
+
+
+def test_a_state_without_log_probabilities():
+    """``sample`` needs the configurations alone, as ``reset`` does."""
+    import netket_gb300 as nk
+    hi = nk.hilbert.Spin(0.5, 6)
+    vs = _state(nk, nk.sampler.MetropolisLocal(hi, n_chains=8), 2)
+    vs.sampler_state.log_prob = None
+    vs.sample()
+    st = vs.sampler_state
+    torch.testing.assert_close(st.log_prob, 2.0 * vs.log_value(st.σ), rtol=1e-12, atol=1e-12)
